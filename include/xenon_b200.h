@@ -449,10 +449,10 @@ typedef struct xb_tuning {
                                            16 blocks of 128 threads per SM: fewer registers per
                                            thread, the rest spilled to L1 (other values: 8; the
                                            guided bounces take 4 or 8, 8 for 12 and 16) */
-  int32_t shared_stack;                 /* traversal kernels: 16 = the first 16 entries of each
-                                           thread's BLAS stack in shared memory (8 KB per block of
-                                           128 threads), the rest in local memory; 1 (default, and
-                                           any other value): all in local memory. Same hits. */
+  int32_t shared_stack;                 /* traversal kernels: 16 = the first 16 words of each
+                                           thread's traversal stack in shared memory (8 KB per block
+                                           of 128 threads), the rest in local memory; 1 (default,
+                                           and any other value): all in local memory. Same hits. */
   int32_t pixel_order;                  /* camera rays in the queue: 1 scanline order, 2 (default)
                                            each warp's 32 rays from one 8x4 pixel tile (config 3:
                                            5 % faster). Same image either way. */

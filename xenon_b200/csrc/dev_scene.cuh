@@ -1,16 +1,20 @@
 // dev_scene.cuh — the scene as laid out in HBM, and its traversal.
 //
 // Layout (all read-only, loaded through the non-coherent path):
-//   blas      float4[2 * N]: node i = {mn.x, mn.y, mn.z, mx.x}, {mx.y, mx.z, child, count}.
-//             All meshes' BLAS arrays are concatenated; each mesh's nodes start at an odd
-//             index so that every child pair (left, left+1) is one 64-byte aligned block:
-//             an internal node costs one 64 B pair load, as in the reference's two-child
-//             test (src/geometry/blas.cpp:103-152). child fields are global indices.
+//   nodes     float4[2 * N]: node i = {mn.x, mn.y, mx.x, mx.y}, {mn.z, mx.z, entry, key}. The
+//             TLAS nodes come first, then every mesh's BLAS nodes, each mesh starting at an odd
+//             index so that a child pair (left, left+1) is one 64-byte block: expanding a node
+//             costs one 64 B pair load (two 256-bit loads), as in the reference's two-child test
+//             (src/geometry/blas.cpp:103-152). entry is the node as the traversal stacks it (see
+//             kLeafEntry). The order of the six planes makes each register pair of the load an
+//             operand of the packed (f32x2) slab arithmetic. key: a BLAS node's triangle count
+//             (the refit reads it), a TLAS node's centre on its parent's widest axis.
 //   tris      float4[3 * S]: the triangle of BLAS prim slot s, pre-gathered in slot order
 //             {v0, local tri id}, {v1, global tri id}, {v2, -}: a leaf's triangles are
 //             contiguous 48 B records (src/geometry/mesh.h:37-44 gather, done once on upload).
 //   pnodes    the PrimBLAS nodes, same 32 B records; prims the analytic primitives.
-//   tlas      TLAS nodes, 32 B each; inst the instances (world_to_local + BLAS root).
+//   inst      the instances (world_to_local + BLAS root) in the order the TLAS leaves list them,
+//             so a leaf's instances are contiguous.
 //
 // Traversal restates the reference's order and float semantics exactly:
 //   BLAS closest / any       src/geometry/blas.cpp:211-307 (+ aabb_pair_sse :25-74)
@@ -27,31 +31,40 @@ namespace xbd {
 
 constexpr int kStackSize = 64;   // BLAS / TLAS / PrimBLAS stacks are 64 deep in the reference
 constexpr int kShStride = 128;   // threads per block of every traversal kernel
-constexpr int kSharedStack = 16; // BLAS stack entries the shared-stack kernels keep in shared memory
+constexpr int kSharedStack = 16; // stack entries the shared-stack kernels keep in shared memory
 
-// The BLAS / PrimBLAS traversal stack. Its first NSH entries live in shared memory (entry k of
-// thread t at sh[k * kShStride + t]: a warp's 32 accesses fall in 32 distinct banks at any mix of
-// depths), the rest in the thread's local array (entries k >= NSH at loc[k]). NSH = 0 keeps the
-// whole stack in local memory and compiles to plain local-array accesses.
-template <int NSH>
-struct BStack {
-  uint32_t* sh;
-  uint32_t* loc;
-  __device__ __forceinline__ uint32_t get(int k) const {
+// The traversal stack: a ray's TLAS entries, above them those of the BLAS it is in. Its first NSH
+// entries live in shared memory (entry k of thread t at sh[k * kShStride + t]: a warp's accesses
+// fall in distinct banks at any mix of depths), the rest in the thread's local array (entries
+// k >= NSH at loc[k]). NSH = 0 keeps the whole stack in local memory and compiles to plain
+// local-array accesses.
+template <class Entry, int NSH>
+struct TStack {
+  Entry* sh;
+  Entry* loc;
+  __device__ __forceinline__ Entry get(int k) const {
     if constexpr (NSH == 0) return loc[k];
     else return k < NSH ? sh[k * kShStride] : loc[k];
   }
-  __device__ __forceinline__ void put(int k, uint32_t v) const {
+  __device__ __forceinline__ void put(int k, Entry v) const {
     if constexpr (NSH == 0) loc[k] = v;
     else if (k < NSH) sh[k * kShStride] = v;
     else loc[k] = v;
   }
 };
+// The PrimBLAS walk's own stack, above the `base` words of a traversal stack.
+template <class Stack>
+struct StackAbove {
+  Stack st;
+  int base;
+  __device__ __forceinline__ uint32_t get(int k) const { return st.get(base + k); }
+  __device__ __forceinline__ void put(int k, uint32_t v) const { st.put(base + k, v); }
+};
 
-struct DevInstance {     // 64 bytes
+struct alignas(32) DevInstance {   // 64 bytes
   float w2l[12];         // world_to_local, columns c0 c1 c2 c3
   int32_t kind;          // 0 = triangle BLAS, 1 = prim BLAS
-  int32_t root;          // global index of the BLAS root node
+  uint32_t root;         // the BLAS root node's entry
   int32_t instance_id;
   int32_t mesh;          // mesh index (kind 0)
 };
@@ -90,12 +103,11 @@ struct DevMesh {
 };
 
 struct DevScene {
-  const float4* blas;
+  const float4* nodes;
   const float4* tris;
+  const uint2* big_leaves;   // (first, count) of the leaves that an entry cannot hold
   const float4* pnodes;
   const float4* prims;       // 4 float4 per prim slot: {type, mat, prim index, -}, p0..p3, p4..p7, p8 p9
-  const float4* tlas;
-  const uint32_t* tlas_inst;
   const DevInstance* inst;
   const DevMesh* meshes;
   const int32_t* tri_index;  // 3 global vertex ids per global triangle
@@ -116,6 +128,8 @@ struct DevScene {
   int32_t sun_nee;   // XB_FLAG_SUN_NEE: directional lights weighted as delta lights (else the reference's 1e8)
   const float* sky_cdf;   // XB_FLAG_SKY_IS: kSkyBins + 1 cumulative bin masses over y in [-1, 1] (or nullptr)
   int32_t watertight;     // XB_FLAG_WATERTIGHT: ray_triangle_wt instead of Moller-Trumbore
+  float4 root_a, root_b;  // the TLAS root, as in nodes
+  int32_t loose_boxes;    // some box holds a NaN, or a TLAS box is inverted: every ray is `odd` (SlabRay)
 };
 
 // The sky's luminance distribution over directions. The gradient sky (Environment::evaluate)
@@ -154,7 +168,7 @@ struct Ray {
 struct HitState {
   float t, u, v;
   int32_t prim;    // triangle: BLAS slot; analytic: prim index
-  int32_t inst;    // instance index (-1: no hit)
+  int32_t inst;    // index into DevScene::inst (-1: no hit)
 };
 
 struct TraversalCounters {
@@ -166,27 +180,35 @@ struct TraversalCounters {
 
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
 
-// BLAS stack entries carry the node's own (child, count) — both already loaded with the
-// parent's 64 B child pair — so popping needs no further node load: count in the top 4 bits,
-// child (a node or triangle-slot index < 2^28) below. A count >= 15 (only degenerate leaves)
-// stores the node index instead, marked by 15, and the node is re-read when popped.
+// 32 bytes, 32-byte aligned, in one 256-bit load (sm_100): half the load instructions and L1
+// lookups of two float4 loads for lanes that read scattered nodes.
+__device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
+// A node as the traversal stacks it: its (child, count), already loaded with the parent's 64 B
+// child pair, so popping needs no further node load. In a BLAS: count in the top 4 bits, child (a
+// node or triangle-slot index < 2^28) below. In the TLAS the low 28 bits are child << 1 (a node
+// or instance index < 2^27) and a bit of the pair's ordering axis, bit 0 of the axis in the left
+// child's entry and bit 1 in the right one's. A count of 15 or more (only degenerate leaves), or an
+// instance index that does not fit, has 15 above and a place in DevScene::big_leaves instead of
+// the child. Entries are packed once, at upload (renderer.cu). kNoWork and kDone are entries of no
+// node: that table is far shorter than 2^27.
 constexpr uint32_t kEntryEscape = 15u;
-__device__ __forceinline__ uint32_t blas_entry(uint32_t child, uint32_t count, uint32_t node) {
-  return count < kEntryEscape ? ((count << 28) | child) : ((kEntryEscape << 28) | node);
-}
-__device__ __forceinline__ void blas_unpack(const DevScene& sc, uint32_t e, uint32_t& child,
-                                            uint32_t& count) {
+constexpr uint32_t kLeafEntry = 1u << 28;         // entries below: interior nodes
+constexpr uint32_t kNoWork = 0xffffffffu;
+constexpr uint32_t kDone = 0xfffffffeu;
+__device__ __forceinline__ void leaf_unpack(const DevScene& sc, uint32_t e, uint32_t& first, uint32_t& count,
+                                            int shift = 0) {
   count = e >> 28;
-  child = e & 0x0fffffffu;
+  first = (e & (kLeafEntry - 1u)) >> shift;
   if (count == kEntryEscape) {
-    const float4 nb = __ldg(sc.blas + 2 * (size_t)child + 1);
-    child = __float_as_uint(nb.z);
-    count = __float_as_uint(nb.w);
+    const uint2 l = __ldg(sc.big_leaves + first);
+    first = l.x;
+    count = l.y;
   }
-}
-__device__ __forceinline__ uint32_t blas_root_entry(const DevScene& sc, int root) {
-  const float4 nb = __ldg(sc.blas + 2 * (size_t)root + 1);
-  return blas_entry(__float_as_uint(nb.z), __float_as_uint(nb.w), (uint32_t)root);
 }
 
 // ── world → local (AffineTransform::to_local, transform.h:44-51) ────────────────
@@ -200,6 +222,14 @@ __device__ __forceinline__ Ray to_local(const DevInstance& in, const Ray& w) {
   r.tmin = w.tmin;
   r.tmax = w.tmax;
   return r;
+}
+
+// One instance through 256-bit loads.
+__device__ __forceinline__ DevInstance load_instance(const DevInstance* p) {
+  union { DevInstance in; float4 q[4]; } u;
+  ldg8(reinterpret_cast<const float4*>(p), u.q[0], u.q[1]);
+  ldg8(reinterpret_cast<const float4*>(p) + 2, u.q[2], u.q[3]);
+  return u.in;
 }
 
 // normal_to_world: normalize(world_to_local.transform_normal(n)) (transform.h:41-45, 56-58)
@@ -284,10 +314,10 @@ __device__ __forceinline__ float mmax(float a, float b) { return a > b ? a : b; 
 // aabb_pair_sse for one child: returns near t via tn, hit flag
 __device__ __forceinline__ bool slab_sse(float4 a, float4 b, V3 inv, V3 org, float tmin,
                                          float tmax, float& tn) {
-  // a = {mn.x, mn.y, mn.z, mx.x}, b = {mx.y, mx.z, ...}
-  float t0x = (a.x - org.x) * inv.x, t1x = (a.w - org.x) * inv.x;
-  float t0y = (a.y - org.y) * inv.y, t1y = (b.x - org.y) * inv.y;
-  float t0z = (a.z - org.z) * inv.z, t1z = (b.y - org.z) * inv.z;
+  // a = {mn.x, mn.y, mx.x, mx.y}, b = {mn.z, mx.z, ...}
+  float t0x = (a.x - org.x) * inv.x, t1x = (a.z - org.x) * inv.x;
+  float t0y = (a.y - org.y) * inv.y, t1y = (a.w - org.y) * inv.y;
+  float t0z = (b.x - org.z) * inv.z, t1z = (b.y - org.z) * inv.z;
   float lx = mmin(t0x, t1x), ly = mmin(t0y, t1y), lz = mmin(t0z, t1z);
   float hx = mmax(t0x, t1x), hy = mmax(t0y, t1y), hz = mmax(t0z, t1z);
   float tnear = mmax(mmax(mmax(lx, ly), lz), tmin);
@@ -296,16 +326,48 @@ __device__ __forceinline__ bool slab_sse(float4 a, float4 b, V3 inv, V3 org, flo
   return tnear <= tfar;
 }
 
-// AABB::intersect_fast (aabb.h:59-71) with std::max/min over initializer lists
-__device__ __forceinline__ bool aabb_fast(float4 a, float4 b, V3 inv, V3 org, const int sign[3],
-                                          float tmin, float tmax) {
-  float mnx = a.x, mny = a.y, mnz = a.z, mxx = a.w, mxy = b.x, mxz = b.y;
-  float txmin = ((sign[0] ? mxx : mnx) - org.x) * inv.x;
-  float txmax = ((sign[0] ? mnx : mxx) - org.x) * inv.x;
-  float tymin = ((sign[1] ? mxy : mny) - org.y) * inv.y;
-  float tymax = ((sign[1] ? mny : mxy) - org.y) * inv.y;
-  float tzmin = ((sign[2] ? mxz : mnz) - org.z) * inv.z;
-  float tzmax = ((sign[2] ? mnz : mxz) - org.z) * inv.z;
+// Packed pairs (sm_100 add / mul.f32x2): each half rounds as the scalar instruction does.
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 a, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// AABB::intersect_fast (aabb.h:59-71) with std::max/min over initializer lists; tn: the larger of
+// tmin and the entry distances
+__device__ __forceinline__ bool aabb_fast(float4 a, float4 b, V3 inv, V3 org, V3 dir, float tmin, float tmax,
+                                          float& tn) {
+  const bool sx = dir.x < 0.f, sy = dir.y < 0.f, sz = dir.z < 0.f;
+  float txmin = ((sx ? a.z : a.x) - org.x) * inv.x;
+  float txmax = ((sx ? a.x : a.z) - org.x) * inv.x;
+  float tymin = ((sy ? a.w : a.y) - org.y) * inv.y;
+  float tymax = ((sy ? a.y : a.w) - org.y) * inv.y;
+  float tzmin = ((sz ? b.y : b.x) - org.z) * inv.z;
+  float tzmax = ((sz ? b.x : b.y) - org.z) * inv.z;
   float lo = tmin;
   if (lo < txmin) lo = txmin;
   if (lo < tymin) lo = tymin;
@@ -314,8 +376,56 @@ __device__ __forceinline__ bool aabb_fast(float4 a, float4 b, V3 inv, V3 org, co
   if (txmax < hi) hi = txmax;
   if (tymax < hi) hi = tymax;
   if (tzmax < hi) hi = tzmax;
+  tn = lo;
   return lo <= hi;
 }
+
+// A ray's slab operands in the space of the nodes it is among. slab() gives the hit flag and near
+// t of slab_sse (BLAS pairs) and of aabb_fast (TLAS nodes) from the same differences and products
+// (a - o is a + (-o), in packed pairs) through the hardware's minimum and maximum. Those differ
+// from minps / maxps only in which operand a NaN leaves and in the sign of a zero; a comparison
+// reads both zeros alike, and no NaN arises while 1 / d is finite and not zero, the origin is
+// finite, tmin and tmax are not NaN and the boxes hold no NaN: 0 * inf and inf - inf are ruled out.
+// With boxes that are not inverted the smaller of a slab's two distances is also the one that
+// aabb_fast picks by the direction's sign. A ray of which any of that is not so (an axis-parallel
+// direction, for one) is `odd` and takes the reference's forms.
+struct SlabRay {
+  F2 noxy, noz, ixy, iz;
+  __device__ __forceinline__ void set(V3 o, V3 inv) {
+    noxy = f2(-o.x, -o.y);
+    noz = f2(-o.z, -o.z);
+    ixy = f2(inv.x, inv.y);
+    iz = f2(inv.z, inv.z);
+  }
+  static __device__ __forceinline__ bool odd(const DevScene& sc, V3 o, V3 inv, float tmin, float tmax) {
+    // x - x is 0 for finite x, else NaN
+    const float fin = (inv.x - inv.x) + (inv.y - inv.y) + (inv.z - inv.z) + (o.x - o.x) + (o.y - o.y) + (o.z - o.z);
+    return !(fin == 0.f && tmin == tmin && tmax == tmax && inv.x != 0.f && inv.y != 0.f && inv.z != 0.f) ||
+           sc.loose_boxes != 0;
+  }
+  __device__ __forceinline__ V3 norg() const {   // -origin
+    float x, y, z, w;
+    unpack2(noxy, x, y);
+    unpack2(noz, z, w);
+    return v3(x, y, z);
+  }
+  __device__ __forceinline__ V3 org() const { return -norg(); }
+  __device__ __forceinline__ V3 inv() const {
+    float x, y, z, w;
+    unpack2(ixy, x, y);
+    unpack2(iz, z, w);
+    return v3(x, y, z);
+  }
+  __device__ __forceinline__ bool slab(float4 a, float4 b, float tmin, float tmax, float& tn) const {
+    float t0x, t0y, t1x, t1y, t0z, t1z;
+    unpack2(mul2(add2(f2(a.x, a.y), noxy), ixy), t0x, t0y);
+    unpack2(mul2(add2(f2(a.z, a.w), noxy), ixy), t1x, t1y);
+    unpack2(mul2(add2(f2(b.x, b.y), noz), iz), t0z, t1z);
+    tn = fmaxf(max3(fminf(t0x, t1x), fminf(t0y, t1y), fminf(t0z, t1z)), tmin);
+    const float tf = fminf(min3(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z)), tmax);
+    return tn <= tf;
+  }
+};
 
 // AABB::intersect (aabb.h:41-56): division slabs, std::max / std::min folds
 __device__ __forceinline__ bool aabb_div(float4 a, float4 b, const Ray& r, float& tn) {
@@ -419,106 +529,6 @@ __device__ __forceinline__ bool prim_intersect(const float4* pr, const Ray& r, f
   }
 }
 
-// ── BLAS closest hit (blas.cpp:211-265) ──────────────────────────────────────────
-template <bool kCount, class Stack>
-__device__ __forceinline__ bool blas_closest(const DevScene& sc, int root, const Ray& r,
-                                             HitState& h, int inst_idx, const Stack& stack,
-                                             TraversalCounters& cnt, bool& overflow) {
-  // The reference pushes (far, near) and pops near at once; here the near child continues in
-  // a register and only the far one is pushed: the same visit order, half the stack traffic.
-  const V3 inv = v3(1.f / r.d.x, 1.f / r.d.y, 1.f / r.d.z);
-  int ptr = 0;
-  uint32_t cur = blas_root_entry(sc, root);
-  bool hit = false;
-  for (;;) {
-    uint32_t child, count;
-    blas_unpack(sc, cur, child, count);
-    if (count > 0) {
-      for (uint32_t i = 0; i < count; ++i) {
-        const float4* tp = sc.tris + 3 * (size_t)(child + i);
-        const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
-        if (kCount) cnt.tris++;
-        float t, u, v;
-        if (tri_hit(sc, r.o, r.d, inv, r.tmin, ld3(a), ld3(b), ld3(c), h.t, t, u, v)) {
-          h.t = t; h.u = u; h.v = v;
-          h.prim = (int32_t)(child + i);
-          h.inst = inst_idx;
-          hit = true;
-        }
-      }
-      if (ptr == 0) break;
-      cur = stack.get(--ptr);
-      continue;
-    }
-    if (kCount) cnt.nodes++;
-    const float4* pp = sc.blas + 2 * (size_t)child;
-    const float4 la = ldg4(pp), lb = ldg4(pp + 1), ra = ldg4(pp + 2), rb = ldg4(pp + 3);
-    float tl, tr;
-    const bool hl = slab_sse(la, lb, inv, r.o, r.tmin, h.t, tl);
-    const bool hr = slab_sse(ra, rb, inv, r.o, r.tmin, h.t, tr);
-    const uint32_t el = blas_entry(__float_as_uint(lb.z), __float_as_uint(lb.w), child);
-    const uint32_t er = blas_entry(__float_as_uint(rb.z), __float_as_uint(rb.w), child + 1);
-    if (hl && hr) {
-      if (ptr + 1 > kStackSize) { overflow = true; break; }
-      if (tl < tr) { stack.put(ptr++, er); cur = el; }
-      else { stack.put(ptr++, el); cur = er; }
-    } else if (hl || hr) {
-      cur = hl ? el : er;
-    } else {
-      if (ptr == 0) break;
-      cur = stack.get(--ptr);
-    }
-  }
-  return hit;
-}
-
-// ── BLAS any hit (blas.cpp:269-307) ──────────────────────────────────────────────
-template <bool kCount, class Stack>
-__device__ __forceinline__ bool blas_any(const DevScene& sc, int root, const Ray& r,
-                                         const Stack& stack, TraversalCounters& cnt, bool& overflow,
-                                         bool far_first = false) {
-  // Whether some triangle lies in [tmin, tmax] does not depend on the visit order, so the order
-  // is a tuning choice: nearest child first, or farthest first (shadow rays start on a surface,
-  // where their occluder rarely is).
-  const V3 inv = v3(1.f / r.d.x, 1.f / r.d.y, 1.f / r.d.z);
-  int ptr = 0;
-  uint32_t cur = blas_root_entry(sc, root);
-  for (;;) {
-    uint32_t child, count;
-    blas_unpack(sc, cur, child, count);
-    if (count > 0) {
-      for (uint32_t i = 0; i < count; ++i) {
-        const float4* tp = sc.tris + 3 * (size_t)(child + i);
-        const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
-        if (kCount) cnt.tris++;
-        float t, u, v;
-        if (tri_hit(sc, r.o, r.d, inv, r.tmin, ld3(a), ld3(b), ld3(c), r.tmax, t, u, v)) return true;
-      }
-      if (ptr == 0) return false;
-      cur = stack.get(--ptr);
-      continue;
-    }
-    if (kCount) cnt.nodes++;
-    const float4* pp = sc.blas + 2 * (size_t)child;
-    const float4 la = ldg4(pp), lb = ldg4(pp + 1), ra = ldg4(pp + 2), rb = ldg4(pp + 3);
-    float tl, tr;
-    const bool hl = slab_sse(la, lb, inv, r.o, r.tmin, r.tmax, tl);
-    const bool hr = slab_sse(ra, rb, inv, r.o, r.tmin, r.tmax, tr);
-    const uint32_t el = blas_entry(__float_as_uint(lb.z), __float_as_uint(lb.w), child);
-    const uint32_t er = blas_entry(__float_as_uint(rb.z), __float_as_uint(rb.w), child + 1);
-    if (hl && hr) {
-      if (ptr + 1 > kStackSize) { overflow = true; return false; }
-      if ((tl < tr) != far_first) { stack.put(ptr++, er); cur = el; }
-      else { stack.put(ptr++, el); cur = er; }
-    } else if (hl || hr) {
-      cur = hl ? el : er;
-    } else {
-      if (ptr == 0) return false;
-      cur = stack.get(--ptr);
-    }
-  }
-}
-
 // ── PrimBLAS closest hit (prim_blas.cpp:142-194) ───────────────────────────────
 template <class Stack>
 __device__ __forceinline__ bool pblas_closest(const DevScene& sc, const Ray& r, HitState& h,
@@ -589,89 +599,6 @@ __device__ __forceinline__ bool pblas_any(const DevScene& sc, const Ray& r, cons
   return false;
 }
 
-// ── TLAS closest hit (tlas.cpp:172-245) ──────────────────────────────────────────
-template <bool kCount, class Stack>
-__device__ __forceinline__ bool scene_closest(const DevScene& sc, const Ray& w, HitState& h,
-                                              uint32_t* tstack, const Stack& bstack,
-                                              TraversalCounters& cnt, bool& overflow) {
-  h.t = kInf; h.u = 0.f; h.v = 0.f; h.prim = -1; h.inst = -1;
-  if (sc.num_tlas_nodes == 0) return false;
-  const V3 inv = v3(1.f / w.d.x, 1.f / w.d.y, 1.f / w.d.z);
-  const int sign[3] = {w.d.x < 0.f, w.d.y < 0.f, w.d.z < 0.f};
-  int ptr = 0;
-  tstack[ptr++] = 0;
-  bool hit = false;
-  while (ptr > 0) {
-    const uint32_t idx = tstack[--ptr];
-    const float4 na = ldg4(sc.tlas + 2 * idx), nb = ldg4(sc.tlas + 2 * idx + 1);
-    if (kCount) cnt.tlas++;
-    if (!aabb_fast(na, nb, inv, w.o, sign, w.tmin, h.t)) continue;
-    const uint32_t child = __float_as_uint(nb.z), count = __float_as_uint(nb.w);
-    if (count > 0) {
-      for (uint32_t i = 0; i < count; ++i) {
-        const int ii = (int)__ldg(sc.tlas_inst + child + i);
-        const DevInstance& in = sc.inst[ii];
-        if (kCount) cnt.inst++;
-        const Ray lr = to_local(in, w);
-        bool got;
-        if (in.kind == 0) got = blas_closest<kCount>(sc, in.root, lr, h, ii, bstack, cnt, overflow);
-        else got = pblas_closest(sc, lr, h, ii, bstack, overflow);
-        hit |= got;
-      }
-      continue;
-    }
-    // order by the children's centre projections on the parent's widest axis
-    const float ex = na.w - na.x, ey = nb.x - na.y, ez = nb.y - na.z;
-    const int ax = (ex > ey && ex > ez) ? 0 : (ey > ez ? 1 : 2);
-    const float4 la = ldg4(sc.tlas + 2 * child), lb = ldg4(sc.tlas + 2 * child + 1);
-    const float4 ra = ldg4(sc.tlas + 2 * child + 2), rb = ldg4(sc.tlas + 2 * child + 3);
-    float cl, cr;
-    if (ax == 0) { cl = (la.x + la.w) * 0.5f; cr = (ra.x + ra.w) * 0.5f; }
-    else if (ax == 1) { cl = (la.y + lb.x) * 0.5f; cr = (ra.y + rb.x) * 0.5f; }
-    else { cl = (la.z + lb.y) * 0.5f; cr = (ra.z + rb.y) * 0.5f; }
-    const float tl = (cl - comp(w.o, ax)) * comp(inv, ax);
-    const float tr = (cr - comp(w.o, ax)) * comp(inv, ax);
-    if (ptr + 2 > kStackSize) { overflow = true; break; }
-    if (tl < tr) { tstack[ptr++] = child + 1; tstack[ptr++] = child; }
-    else { tstack[ptr++] = child; tstack[ptr++] = child + 1; }
-  }
-  return hit;
-}
-
-// ── TLAS any hit (tlas.cpp:248-290) ──────────────────────────────────────────────
-template <bool kCount, class Stack>
-__device__ __forceinline__ bool scene_any(const DevScene& sc, const Ray& w, uint32_t* tstack,
-                                          const Stack& bstack, TraversalCounters& cnt, bool& overflow,
-                                          bool far_first = false) {
-  if (sc.num_tlas_nodes == 0) return false;
-  const V3 inv = v3(1.f / w.d.x, 1.f / w.d.y, 1.f / w.d.z);
-  const int sign[3] = {w.d.x < 0.f, w.d.y < 0.f, w.d.z < 0.f};
-  int ptr = 0;
-  tstack[ptr++] = 0;
-  while (ptr > 0) {
-    const uint32_t idx = tstack[--ptr];
-    const float4 na = ldg4(sc.tlas + 2 * idx), nb = ldg4(sc.tlas + 2 * idx + 1);
-    if (kCount) cnt.tlas++;
-    if (!aabb_fast(na, nb, inv, w.o, sign, w.tmin, w.tmax)) continue;
-    const uint32_t child = __float_as_uint(nb.z), count = __float_as_uint(nb.w);
-    if (count > 0) {
-      for (uint32_t i = 0; i < count; ++i) {
-        const DevInstance& in = sc.inst[__ldg(sc.tlas_inst + child + i)];
-        if (kCount) cnt.inst++;
-        const Ray lr = to_local(in, w);
-        const bool got = (in.kind == 0) ? blas_any<kCount>(sc, in.root, lr, bstack, cnt, overflow, far_first)
-                                        : pblas_any(sc, lr, bstack, overflow);
-        if (got) return true;
-      }
-      continue;
-    }
-    if (ptr + 2 > kStackSize) { overflow = true; return false; }
-    tstack[ptr++] = child;
-    tstack[ptr++] = child + 1;
-  }
-  return false;
-}
-
 // ── hit completion: the rest of the HitRecord for the final closest hit ─────────
 struct FullHit {
   V3 pos, normal, geo_normal;
@@ -682,8 +609,7 @@ struct FullHit {
 
 __device__ __forceinline__ void complete_hit(const DevScene& sc, const Ray& w, const HitState& h,
                                              FullHit& f) {
-  const DevInstance& in = sc.inst[h.inst];
-  const Ray lr = to_local(in, w);
+  const DevInstance in = load_instance(sc.inst + h.inst);
   V3 n, gn;
   if (in.kind == 0) {
     // TriangleMesh::intersect_triangle (mesh.h:104-129)
@@ -708,6 +634,7 @@ __device__ __forceinline__ void complete_hit(const DevScene& sc, const Ray& w, c
     f.u = h.u; f.v = h.v;
   } else {
     // the analytic prim's own normal and UV (primitives.h), on the local ray
+    const Ray lr = to_local(in, w);
     const float4* pr = sc.prims + 4 * (size_t)h.prim;
     const float4 h0 = ldg4(pr), h1 = ldg4(pr + 1), h2 = ldg4(pr + 2), h3 = ldg4(pr + 3);
     const int type = __float_as_int(h0.x);

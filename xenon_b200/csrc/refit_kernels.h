@@ -4,11 +4,13 @@
 // the same way). The CPU tests of the host refit therefore run the device refit's pass code.
 //
 // Packed arrays (as xb_upload_scene lays them out):
-//   blas: two quads per node, {mn.x, mn.y, mn.z, mx.x} and {mx.y, mx.z, child, count} with child
-//     and count as bit patterns. An interior node (count 0) has its children at global node
-//     indices child and child + 1; a leaf covers global triangle slots [child, child + count).
+//   blas: two quads per node, {mn.x, mn.y, mx.x, mx.y} and {mn.z, mx.z, entry, count} with entry
+//     and count as bit patterns. child = entry & child_mask, but for leaves of big_count triangles
+//     or more child = big_leaves[2 * (entry & child_mask)]. An interior node (count 0) has its
+//     children at global node indices child and child + 1; a leaf covers global triangle slots
+//     [child, child + count).
 //   tris: three quads per triangle slot, the vertices, with the triangle's index within its mesh
-//     in the first quad's w.
+//     in the first quad's w (the other two w are kept).
 //   tri_index: three global vertex ids per global triangle.
 // Passes:
 //   1. refit_tris_at(s):    slot s takes its vertices from the new positions;
@@ -37,6 +39,8 @@ struct RefitArgs {
   int32_t* parent;            // per node of the mesh: its parent (-1: the root); all -1 at first
   uint32_t* arrivals;         // per node of the mesh: children whose walk reached it
   int32_t* status;            // 0 ok; 1 an index out of range; 2 a walk longer than the node count
+  const uint32_t* big_leaves;
+  uint32_t child_mask, big_count;
   int64_t node_base, slot_base;
   int32_t num_nodes, num_tris, num_verts, tri_offset, vtx_offset;
 };
@@ -68,19 +72,19 @@ XB_HD RefitBox refit_load_box(const Quad* blas, int64_t n) {
   const Quad lo = blas[2 * n], hi = blas[2 * n + 1];
 #endif
   RefitBox b;
-  b.mn[0] = lo.x; b.mn[1] = lo.y; b.mn[2] = lo.z;
-  b.mx[0] = lo.w; b.mx[1] = hi.x; b.mx[2] = hi.y;
+  b.mn[0] = lo.x; b.mn[1] = lo.y; b.mn[2] = hi.x;
+  b.mx[0] = lo.z; b.mx[1] = lo.w; b.mx[2] = hi.y;
   return b;
 }
 
 XB_HD void refit_store_box(Quad* blas, int64_t n, const RefitBox& b, const Quad& hi) {
 #ifdef __CUDA_ARCH__
   float4* p = reinterpret_cast<float4*>(blas) + 2 * n;
-  __stcg(p, make_float4(b.mn[0], b.mn[1], b.mn[2], b.mx[0]));
-  __stcg(p + 1, make_float4(b.mx[1], b.mx[2], hi.z, hi.w));
+  __stcg(p, make_float4(b.mn[0], b.mn[1], b.mx[0], b.mx[1]));
+  __stcg(p + 1, make_float4(b.mn[2], b.mx[2], hi.z, hi.w));
 #else
-  blas[2 * n] = Quad{b.mn[0], b.mn[1], b.mn[2], b.mx[0]};
-  blas[2 * n + 1] = Quad{b.mx[1], b.mx[2], hi.z, hi.w};
+  blas[2 * n] = Quad{b.mn[0], b.mn[1], b.mx[0], b.mx[1]};
+  blas[2 * n + 1] = Quad{b.mn[2], b.mx[2], hi.z, hi.w};
 #endif
 }
 
@@ -118,7 +122,7 @@ XB_HD void refit_parents_at(const RefitArgs& a, int32_t i) {
   a.arrivals[i] = 0u;
   const Quad hi = a.blas[2 * (a.node_base + i) + 1];
   if (quad_bits(hi.w) != 0u) return;   // a leaf
-  const int64_t c = (int64_t)quad_bits(hi.z) - a.node_base;
+  const int64_t c = (int64_t)(quad_bits(hi.z) & a.child_mask) - a.node_base;
   if (c < 1 || c + 1 >= a.num_nodes) { refit_status(a.status, 1); return; }
   a.parent[c] = i;
   a.parent[c + 1] = i;
@@ -128,7 +132,8 @@ XB_HD void refit_nodes_at(const RefitArgs& a, int32_t i) {
   const Quad hi = a.blas[2 * (a.node_base + i) + 1];
   const uint32_t count = quad_bits(hi.w);
   if (count == 0u) return;
-  const int64_t first = quad_bits(hi.z);
+  int64_t first = quad_bits(hi.z) & a.child_mask;
+  if (count >= a.big_count) first = a.big_leaves[2 * first];
   if (first < a.slot_base || first + count > a.slot_base + a.num_tris) { refit_status(a.status, 1); return; }
   const Quad* tris = a.tris;
   auto vertex = [tris](uint32_t slot, int k, float* p) {
@@ -143,7 +148,7 @@ XB_HD void refit_nodes_at(const RefitArgs& a, int32_t i) {
     if (refit_arrive(a.arrivals, p) != 1u) return;    // the first arrival (or a malformed third)
     refit_fence();
     const Quad ph = a.blas[2 * (a.node_base + p) + 1];
-    const int64_t c = quad_bits(ph.z);
+    const int64_t c = quad_bits(ph.z) & a.child_mask;
     refit_store_box(a.blas, a.node_base + p, refit_interior(refit_load_box(a.blas, c), refit_load_box(a.blas, c + 1)),
                     ph);
     i = p;

@@ -73,13 +73,6 @@ enum { STAT_RAYS = 0, STAT_SHADOW = 1, STAT_PATHS = 2, STAT_OVERFLOW = 3,
        STAT_SH_WORK = 12,    // same for shadow rays
        STAT_COUNT = 16 };
 
-__device__ __forceinline__ void flush_counters(unsigned long long* dst, const TraversalCounters& c) {
-  atomicAdd(dst + 0, (unsigned long long)c.nodes);
-  atomicAdd(dst + 1, (unsigned long long)c.tris);
-  atomicAdd(dst + 2, (unsigned long long)c.tlas);
-  atomicAdd(dst + 3, (unsigned long long)c.inst);
-}
-
 #define CK(call)                                                                   \
   do {                                                                             \
     cudaError_t e_ = (call);                                                       \
@@ -168,7 +161,7 @@ struct xb_renderer {
   int refill = 8;                // persistent traversal: refill a warp when this many lanes idle
   int ext_persistent_from = 0;   // bounces >= this trace closest hits with persistent warps
   bool shadow_persistent = true;
-  int occ_ext = 1, occ_pext = 1, occ_shadow = 1, occ_pshadow = 1;  // limits
+  int occ_pext = 1, occ_pshadow = 1;  // blocks of the persistent kernels that fit on an SM at once
   int occ_api[2] = {1, 1};   // trace_api_persistent_kernel<closest / any>
   int stack_sh = 0;             // BLAS stack entries in shared memory (tuning shared_stack)
   xb_tuning tune{};
@@ -201,10 +194,13 @@ struct xb_renderer {
   };
   std::vector<MeshLayout> mesh_layout;
   std::vector<int32_t> inst_geom;
+  std::vector<DevInstance> inst_dev;      // the uploaded instances, by instance index
   std::vector<xb::Affine> inst_l2w;
   xb_bvh_node prim_root{};
   bool has_prim_root = false;
-  int64_t tlas_cap = 0;         // nodes the device TLAS array holds
+  int64_t tlas_cap = 0;         // TLAS nodes that fit at the front of the device's node array
+  int64_t big_leaves = 0;       // entries of its big_leaves
+  bool loose_blas = false;      // see DevScene::loose_boxes
   void* refit_mem = nullptr;
   size_t refit_bytes = 0;
 };
@@ -298,86 +294,13 @@ __global__ void raygen_kernel(CamDev cam, int W, int H, int spp_first, int64_t p
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt[CNT_RAYS] = (int32_t)paths;
 }
 
-// ── extend: closest hit of the bounce's ray queue ─────────────────────────────
-template <bool kCount, int kSh>
-__global__ void __launch_bounds__(128) extend_kernel(DevScene sc, const float4* __restrict__ ray_o,
-                                                     const float4* __restrict__ ray_d,
-                                                     float4* hit, int32_t* hit_inst, int32_t* cnt,
-                                                     unsigned long long* stats) {
-  __shared__ int s_base[4];
-  const int n = cnt[CNT_RAYS];
-  uint32_t tstack[kStackSize];
-  uint32_t bstack_local[kStackSize];
-  extern __shared__ uint32_t s_stack[];
-  const BStack<kSh> bstack{s_stack + threadIdx.x, bstack_local};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  bool overflow = false;
-  TraversalCounters tc{0, 0, 0, 0};
-  for (;;) {
-    if (lane == 0) s_base[warp] = atomicAdd(cnt + CNT_FETCH_EXT, 32);
-    __syncwarp();
-    const int base = s_base[warp];
-    __syncwarp();
-    if (base >= n) break;
-    const int i = base + lane;
-    if (i < n) {
-      const float4 o = ray_o[i], d = ray_d[i];
-      Ray r{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, d.w};
-      HitState h;
-      scene_closest<kCount>(sc, r, h, tstack, bstack, tc, overflow);
-      hit[i] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
-      hit_inst[i] = h.inst;
-    }
-  }
-  if (overflow) atomicAdd(stats + STAT_OVERFLOW, 1ull);
-  if (kCount) flush_counters(stats + STAT_EXT_WORK, tc);
-}
-
-// ── shadow: any hit; unoccluded items add their contribution ──────────────────
-template <bool kCount, int kSh>
-__global__ void __launch_bounds__(128) shadow_kernel(DevScene sc, const float4* __restrict__ so,
-                                                     const float4* __restrict__ sd,
-                                                     const float4* __restrict__ scn, float4* L,
-                                                     const int32_t* count, int32_t* fetch,
-                                                     unsigned long long* stats, int far_first) {
-  __shared__ int s_base[4];
-  const int n = *count;
-  uint32_t tstack[kStackSize];
-  uint32_t bstack_local[kStackSize];
-  extern __shared__ uint32_t s_stack[];
-  const BStack<kSh> bstack{s_stack + threadIdx.x, bstack_local};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  bool overflow = false;
-  TraversalCounters tc{0, 0, 0, 0};
-  for (;;) {
-    if (lane == 0) s_base[warp] = atomicAdd(fetch, 32);
-    __syncwarp();
-    const int base = s_base[warp];
-    __syncwarp();
-    if (base >= n) break;
-    const int i = base + lane;
-    if (i < n) {
-      const float4 o = so[i], d = sd[i];
-      Ray r{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kShadowEps, o.w};
-      if (!scene_any<kCount>(sc, r, tstack, bstack, tc, overflow, far_first != 0)) {
-        const float4 c = scn[i];
-        const int p = __float_as_int(d.w);
-        float4 l = L[p];
-        l.x = l.x + c.x; l.y = l.y + c.y; l.z = l.z + c.z;
-        L[p] = l;
-      }
-    }
-  }
-  if (overflow) atomicAdd(stats + STAT_OVERFLOW, 1ull);
-  if (kCount) flush_counters(stats + STAT_SH_WORK, tc);
-}
-
-// ── persistent-warp variants (trace_persistent.cuh) ────────────────────────────
+// ── extend: closest hit of the bounce's ray queue (trace_persistent.cuh) ──────────
 template <bool kCount, int kSh>
 __global__ void __launch_bounds__(128) extend_persistent_kernel(DevScene sc, TraceQueue q, int refill) {
   QueueIO io{q, *q.count};
   trace_persistent<false, kCount, kSh>(sc, io, refill, false);
 }
+// ── shadow: any hit; unoccluded items add their contribution ──────────────────
 template <bool kCount, int kSh>
 __global__ void __launch_bounds__(128) shadow_persistent_kernel(DevScene sc, TraceQueue q, int refill) {
   QueueIO io{q, *q.count};
@@ -1227,51 +1150,15 @@ __global__ void resolve_kernel(const float4* accum, int W, int H, float inv_spp,
 }
 
 // ── ray queries (xb_trace_rays) ─────────────────────────────────────────────────
-__global__ void __launch_bounds__(128) trace_full_kernel(DevScene sc, const xb_ray* rays,
-                                                         int64_t n, xb_hit* hits, int mode,
-                                                         unsigned long long* stats) {
-  uint32_t tstack[kStackSize];
-  uint32_t bstack_local[kStackSize];
-  const BStack<0> bstack{nullptr, bstack_local};
-  bool overflow = false;
-  TraversalCounters tc{0, 0, 0, 0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const xb_ray rr = rays[i];
-    Ray r{v3(rr.org[0], rr.org[1], rr.org[2]), v3(rr.dir[0], rr.dir[1], rr.dir[2]), rr.tmin, rr.tmax};
-    xb_hit out;
-    memset(&out, 0, sizeof(out));
-    out.t = kInf; out.prim_id = -1; out.instance_id = -1; out.mat_id = -1;
-    if (mode == XB_TRACE_CLOSEST) {
-      HitState h;
-      if (scene_closest<true>(sc, r, h, tstack, bstack, tc, overflow)) {
-        FullHit f;
-        complete_hit(sc, r, h, f);
-        out.t = h.t; out.u = f.u; out.v = f.v;
-        out.prim_id = f.prim_id; out.instance_id = f.instance_id; out.mat_id = f.mat_id;
-        out.front_face = f.front_face ? 1 : 0;
-        out.pos[0] = f.pos.x; out.pos[1] = f.pos.y; out.pos[2] = f.pos.z;
-        out.normal[0] = f.normal.x; out.normal[1] = f.normal.y; out.normal[2] = f.normal.z;
-        out.geo_normal[0] = f.geo_normal.x; out.geo_normal[1] = f.geo_normal.y;
-        out.geo_normal[2] = f.geo_normal.z;
-      }
-    } else {
-      if (scene_any<true>(sc, r, tstack, bstack, tc, overflow)) out.t = 0.f;
-    }
-    hits[i] = out;
-  }
-  if (overflow) atomicAdd(stats + STAT_OVERFLOW, 1ull);
-  flush_counters(stats + (mode == XB_TRACE_CLOSEST ? STAT_EXT_WORK : STAT_SH_WORK), tc);
-}
-
-// xb_trace_rays_device on persistent warps (trace_persistent.cuh): each warp owns a contiguous
-// range of the caller's rays and refills its idle lanes from it, so a long ray no longer holds
-// its warp's finished lanes, and no cursor is shared between calls (calls on different streams
-// may overlap, as with trace_full_kernel). The hit records are trace_full_kernel's.
+// xb_trace_rays_device: each warp owns a contiguous range of the caller's rays and refills its
+// idle lanes from it, so a long ray no longer holds its warp's finished lanes, and no cursor is
+// shared between calls (calls on different streams may overlap).
+// wide: rays and hits are 16-byte aligned (the ABI asks for 4), so records move as float4s.
 struct ApiIO {
   const xb_ray* rays;
   xb_hit* hits;
   unsigned long long* st;
+  bool wide;
   int next, stop;
   __device__ __forceinline__ int end() const { return stop; }
   __device__ __forceinline__ int grab(int, int, int k) {
@@ -1281,6 +1168,15 @@ struct ApiIO {
   }
   template <bool kAny>
   __device__ __forceinline__ void load(int ray, V3& o, V3& d, float& tmin, float& tmax) const {
+    if (wide) {
+      const float4* p = reinterpret_cast<const float4*>(rays + ray);
+      const float4 a = p[0], b = p[1];
+      o = ld3(a);
+      d = ld3(b);
+      tmin = a.w;
+      tmax = b.w;
+      return;
+    }
     const xb_ray rr = rays[ray];
     o = v3(rr.org[0], rr.org[1], rr.org[2]);
     d = v3(rr.dir[0], rr.dir[1], rr.dir[2]);
@@ -1293,10 +1189,21 @@ struct ApiIO {
     out.t = kInf; out.prim_id = -1; out.instance_id = -1; out.mat_id = -1;
     return out;
   }
+  __device__ __forceinline__ void store(int ray, const xb_hit& h) const {
+    if (wide) {
+      float4* p = reinterpret_cast<float4*>(hits + ray);
+      p[0] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim_id));
+      p[1] = make_float4(__int_as_float(h.instance_id), __int_as_float(h.mat_id), __int_as_float(h.front_face), h.pos[0]);
+      p[2] = make_float4(h.pos[1], h.pos[2], h.normal[0], h.normal[1]);
+      p[3] = make_float4(h.normal[2], h.geo_normal[0], h.geo_normal[1], h.geo_normal[2]);
+    } else {
+      hits[ray] = h;
+    }
+  }
   __device__ __forceinline__ void finish_any(int ray, bool occluded) const {
     xb_hit out = miss();
     if (occluded) out.t = 0.f;
-    hits[ray] = out;
+    store(ray, out);
   }
   __device__ __forceinline__ void finish_closest(const DevScene& sc, int ray, V3 o, V3 d, float tmin, float tmax,
                                                  const HitState& h) const {
@@ -1313,7 +1220,7 @@ struct ApiIO {
       out.geo_normal[0] = f.geo_normal.x; out.geo_normal[1] = f.geo_normal.y;
       out.geo_normal[2] = f.geo_normal.z;
     }
-    hits[ray] = out;
+    store(ray, out);
   }
   __device__ __forceinline__ unsigned long long* stats() const { return st; }
 };
@@ -1321,13 +1228,13 @@ struct ApiIO {
 template <bool kAny>
 __global__ void __launch_bounds__(128) trace_api_persistent_kernel(DevScene sc, const xb_ray* rays, int n,
                                                                    xb_hit* hits, unsigned long long* stats,
-                                                                   int refill) {
+                                                                   int refill, bool wide) {
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t chunk = (n + warps - 1) / warps;
   const int64_t b = w * chunk < n ? w * chunk : (int64_t)n;
   const int64_t e = b + chunk < n ? b + chunk : (int64_t)n;
-  ApiIO io{rays, hits, stats, (int)b, (int)e};
+  ApiIO io{rays, hits, stats, wide, (int)b, (int)e};
   trace_persistent<kAny, true, 0>(sc, io, refill, false);
 }
 
@@ -1388,52 +1295,23 @@ __global__ void noalloc_begin_kernel(unsigned long long* scratch, int64_t n) {
   if (threadIdx.x < kNoAllocScratchWords) scratch[threadIdx.x] = threadIdx.x == 1 ? (unsigned long long)n : 0ull;
 }
 
-// Work-stealing variant of trace_full_kernel: warps take 32 rays at a time from the cursor in
-// scratch[0] (ray count in scratch[1]). Threads that overflowed their traversal stack are counted
-// in the renderer's statistics, as trace_full_kernel counts them.
-__global__ void __launch_bounds__(128) trace_stealing_kernel(DevScene sc, const xb_ray* rays, xb_hit* hits,
-                                                             int mode, unsigned long long* scratch,
-                                                             unsigned long long* stats) {
-  __shared__ unsigned long long s_base[4];
-  const int64_t n = (int64_t)scratch[1];
-  uint32_t tstack[kStackSize];
-  uint32_t bstack_local[kStackSize];
-  const BStack<0> bstack{nullptr, bstack_local};
-  bool overflow = false;
-  TraversalCounters tc{0, 0, 0, 0};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (;;) {
-    if (lane == 0) s_base[warp] = atomicAdd(scratch, 32ull);
-    __syncwarp();
-    const int64_t base = (int64_t)s_base[warp];
-    __syncwarp();
-    if (base >= n) break;
-    const int64_t i = base + lane;
-    if (i >= n) continue;
-    const xb_ray rr = rays[i];
-    Ray r{v3(rr.org[0], rr.org[1], rr.org[2]), v3(rr.dir[0], rr.dir[1], rr.dir[2]), rr.tmin, rr.tmax};
-    xb_hit out;
-    memset(&out, 0, sizeof(out));
-    out.t = kInf; out.prim_id = -1; out.instance_id = -1; out.mat_id = -1;
-    if (mode == XB_TRACE_CLOSEST) {
-      HitState h;
-      if (scene_closest<false>(sc, r, h, tstack, bstack, tc, overflow)) {
-        FullHit f;
-        complete_hit(sc, r, h, f);
-        out.t = h.t; out.u = f.u; out.v = f.v;
-        out.prim_id = f.prim_id; out.instance_id = f.instance_id; out.mat_id = f.mat_id;
-        out.front_face = f.front_face ? 1 : 0;
-        out.pos[0] = f.pos.x; out.pos[1] = f.pos.y; out.pos[2] = f.pos.z;
-        out.normal[0] = f.normal.x; out.normal[1] = f.normal.y; out.normal[2] = f.normal.z;
-        out.geo_normal[0] = f.geo_normal.x; out.geo_normal[1] = f.geo_normal.y;
-        out.geo_normal[2] = f.geo_normal.z;
-      }
-    } else if (scene_any<false>(sc, r, tstack, bstack, tc, overflow)) {
-      out.t = 0.f;
-    }
-    hits[i] = out;
+// Warps take rays from the cursor in scratch[0] (ray count in scratch[1]), up to 32 at a time.
+struct NoAllocIO : ApiIO {
+  unsigned long long* cursor;
+  __device__ __forceinline__ int grab(int lane, int leader, int k) const {
+    unsigned long long b = 0;
+    if (lane == leader) b = atomicAdd(cursor, (unsigned long long)k);
+    b = __shfl_sync(0xffffffffu, b, leader);
+    return b < (unsigned long long)stop ? (int)b : stop;
   }
-  if (overflow) atomicAdd(stats + STAT_OVERFLOW, 1ull);
+};
+
+template <bool kAny>
+__global__ void __launch_bounds__(128) trace_stealing_kernel(DevScene sc, const xb_ray* rays, xb_hit* hits,
+                                                             unsigned long long* scratch, unsigned long long* stats,
+                                                             int refill, bool wide) {
+  NoAllocIO io{{rays, hits, stats, wide, 0, (int)scratch[1]}, scratch};
+  trace_persistent<kAny, false, 0>(sc, io, refill, false);
 }
 
 // XB_FLAG_SKY_IS: the sky's luminance (Rec. 709 weights) at the centre of each of kSkyBins bins
@@ -1537,6 +1415,60 @@ int dev_upload(xb_renderer* r, const std::vector<T>& v, const T** out) {
 float4 node_lo(const xb_bvh_node& n) { return make_float4(n.mn[0], n.mn[1], n.mn[2], n.mx[0]); }
 float4 node_hi(const xb_bvh_node& n, uint32_t child) {
   return make_float4(n.mx[1], n.mx[2], u32_bits_to_f(child), u32_bits_to_f(n.count));
+}
+
+// TLAS nodes as DevScene::nodes holds them (entries and keys: dev_scene.cuh). Leaves that an entry
+// cannot hold go to big_leaves, and so do, as empty ones, nodes whose children or instances do not
+// exist. False when a node has two parents (its pair's key would serve one of them) or is the
+// root's parent, or there are too many.
+bool pack_tlas(const xb_bvh_node* nodes, int32_t n, int32_t num_inst, std::vector<float4>& out,
+               std::vector<uint2>& big_leaves, bool& loose) {
+  if (n >= (1 << 27)) return false;
+  std::vector<uint32_t> entry(n);
+  std::vector<float> key(n, 0.f);
+  std::vector<uint8_t> seen(n, 0);
+  if (n > 0) seen[0] = 1;
+  for (int32_t i = 0; i < n; ++i) {
+    const xb_bvh_node& nd = nodes[i];
+    for (int k = 0; k < 3; ++k) loose = loose || !(nd.mn[k] <= nd.mx[k]);
+    const bool leaf = nd.count > 0;
+    const bool exists = leaf ? (int64_t)nd.child + nd.count <= num_inst : (int64_t)nd.child + 1 < n;
+    if (exists && (!leaf || (nd.count < kEntryEscape && nd.child < (1u << 27)))) {
+      entry[i] |= (nd.count << 28) | (nd.child << 1);
+    } else {
+      if (big_leaves.size() >= (1u << 27) - 1) return false;
+      entry[i] |= (kEntryEscape << 28) | ((uint32_t)big_leaves.size() << 1);
+      big_leaves.push_back(exists ? make_uint2(nd.child, nd.count) : make_uint2(0, 0));
+    }
+    if (leaf || !exists) continue;
+    const float ex = nd.mx[0] - nd.mn[0], ey = nd.mx[1] - nd.mn[1], ez = nd.mx[2] - nd.mn[2];
+    const uint32_t ax = (ex > ey && ex > ez) ? 0 : (ey > ez ? 1 : 2);   // tlas.cpp:221-226
+    for (uint32_t c = 0; c < 2; ++c) {
+      const uint32_t ch = nd.child + c;
+      if (seen[ch]) return false;
+      seen[ch] = 1;
+      key[ch] = (nodes[ch].mn[ax] + nodes[ch].mx[ax]) * 0.5f;
+      entry[ch] |= c == 0 ? (ax & 1u) : (ax >> 1);
+    }
+  }
+  out.clear();
+  for (int32_t i = 0; i < n; ++i) {
+    const xb_bvh_node& nd = nodes[i];
+    out.push_back(make_float4(nd.mn[0], nd.mn[1], nd.mx[0], nd.mx[1]));
+    out.push_back(make_float4(nd.mn[2], nd.mx[2], u32_bits_to_f(entry[i]), key[i]));
+  }
+  return true;
+}
+
+// The instances as DevScene::inst holds them; empty when an index is out of range.
+std::vector<DevInstance> in_tlas_order(const std::vector<DevInstance>& insts, const uint32_t* order, size_t n) {
+  std::vector<DevInstance> out;
+  out.reserve(n);
+  for (size_t i = 0; i < n; ++i) {
+    if (order[i] >= insts.size()) return {};
+    out.push_back(insts[order[i]]);
+  }
+  return out;
 }
 
 bool alloc_wave_buffers(WaveBuffers& w, int64_t cap) {
@@ -1726,21 +1658,18 @@ LaneRef lane_ref(xb_renderer* r, int k) {
 // The traversal kernels come in two forms: the BLAS stack wholly in local memory (kSh = 0), or
 // its first kSharedStack entries in shared memory (tuning shared_stack).
 
+// One ray per thread is the same kernel with every lane idle before a refill, on a grid of its own.
 template <int kSh>
 void launch_extend_k(xb_renderer* r, const LaneRef& L, int d, bool count) {
   WaveBuffers& w = *L.w;
   const int q = d & 1;
   int32_t* cd_ = w.cnt + d * kCntStride;
   const size_t smem = (size_t)kSh * kShStride * sizeof(uint32_t);
-  if (r->thread_per_ray || d < r->ext_persistent_from) {
-    auto kern = count ? extend_kernel<true, kSh> : extend_kernel<false, kSh>;
-    kern<<<r->grid_ext, 128, smem, L.s>>>(r->scene, w.ray_o[q], w.ray_d[q], w.hit, w.hit_inst, cd_, r->stats);
-  } else {
-    TraceQueue tq{w.ray_o[q], w.ray_d[q], cd_ + CNT_RAYS, cd_ + CNT_FETCH_EXT, w.hit, w.hit_inst,
-                  nullptr, nullptr, r->stats, 0};
-    auto kern = count ? extend_persistent_kernel<true, kSh> : extend_persistent_kernel<false, kSh>;
-    kern<<<r->grid_pext, 128, smem, L.s>>>(r->scene, tq, r->refill);
-  }
+  const bool per_thread = r->thread_per_ray || d < r->ext_persistent_from;
+  TraceQueue tq{w.ray_o[q], w.ray_d[q], cd_ + CNT_RAYS, cd_ + CNT_FETCH_EXT, w.hit, w.hit_inst,
+                nullptr, nullptr, r->stats, 0};
+  auto kern = count ? extend_persistent_kernel<true, kSh> : extend_persistent_kernel<false, kSh>;
+  kern<<<per_thread ? r->grid_ext : r->grid_pext, 128, smem, L.s>>>(r->scene, tq, per_thread ? 32 : r->refill);
 }
 
 void launch_extend(xb_renderer* r, const LaneRef& L, int d, bool count) {
@@ -1754,19 +1683,12 @@ void launch_shadow_k(xb_renderer* r, const LaneRef& L, int d, int k, bool count,
   WaveBuffers& w = *L.w;
   int32_t* cd_ = w.cnt + d * kCntStride;
   const size_t smem = (size_t)kSh * kShStride * sizeof(uint32_t);
-  if (r->thread_per_ray || !r->shadow_persistent) {
-    auto kern = count ? shadow_kernel<true, kSh> : shadow_kernel<false, kSh>;
-    kern<<<r->grid_shadow, 128, smem, s>>>(r->scene, w.sh_o[k], w.sh_d[k], w.sh_c[k], w.L,
-                                           cd_ + (k ? CNT_SH_SUN : CNT_SH_AREA),
-                                           cd_ + (k ? CNT_FETCH_SH_SUN : CNT_FETCH_SH_AREA), r->stats,
-                                           r->tune.shadow_order == 2);
-  } else {
-    TraceQueue tq{w.sh_o[k], w.sh_d[k], cd_ + (k ? CNT_SH_SUN : CNT_SH_AREA),
-                  cd_ + (k ? CNT_FETCH_SH_SUN : CNT_FETCH_SH_AREA), nullptr, nullptr, w.sh_c[k], w.L,
-                  r->stats, r->tune.shadow_order == 2};
-    auto kern = count ? shadow_persistent_kernel<true, kSh> : shadow_persistent_kernel<false, kSh>;
-    kern<<<r->grid_pshadow, 128, smem, s>>>(r->scene, tq, r->refill);
-  }
+  const bool per_thread = r->thread_per_ray || !r->shadow_persistent;
+  TraceQueue tq{w.sh_o[k], w.sh_d[k], cd_ + (k ? CNT_SH_SUN : CNT_SH_AREA),
+                cd_ + (k ? CNT_FETCH_SH_SUN : CNT_FETCH_SH_AREA), nullptr, nullptr, w.sh_c[k], w.L,
+                r->stats, r->tune.shadow_order == 2};
+  auto kern = count ? shadow_persistent_kernel<true, kSh> : shadow_persistent_kernel<false, kSh>;
+  kern<<<per_thread ? r->grid_shadow : r->grid_pshadow, 128, smem, s>>>(r->scene, tq, per_thread ? 32 : r->refill);
 }
 
 void launch_shadows(xb_renderer* r, const LaneRef& L, int d, bool count, cudaStream_t s) {
@@ -2227,10 +2149,6 @@ int xb_create(const xb_config* cfg, xb_renderer** out) {
   }
   int rc = XB_OK;
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extend_kernel<false, 0>, 128, 0);
-  r->occ_ext = std::max(occ, 1);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shadow_kernel<false, 0>, 128, 0);
-  r->occ_shadow = std::max(occ, 1);
   // guided shade: dynamic shared memory for the weights, one activation tile and the lobes; at
   // most 4 CTAs per SM so their TMEM (64 columns each) always fits the SM's 512 columns
   if (cudaFuncSetAttribute(guide_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2350,6 +2268,22 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   std::vector<DevMesh> meshes(v->num_meshes);
   r->mesh_layout.assign(v->num_meshes, xb_renderer::MeshLayout());
   int64_t slot_base = 0, tri_base = 0, vtx_base = 0;
+  // the TLAS nodes' places at the front; a refit's TLAS has at most two nodes per instance
+  const int64_t tlas_cap = std::max<int64_t>(v->num_tlas_nodes, 2 * (int64_t)v->num_instances);
+  blas.resize(2 * (size_t)tlas_cap, make_float4(0, 0, 0, 0));
+  bool loose = false;
+  std::vector<uint2> big_leaves;
+  size_t nn = 0, nt = 0, nv = 0;
+  for (int m = 0; m < v->num_meshes; ++m) {
+    nn += std::max(v->meshes[m].num_blas_nodes, 0) + 2;
+    nt += std::max(v->meshes[m].num_triangles, 0);
+    nv += std::max(v->meshes[m].num_vertices, 0);
+  }
+  blas.reserve(blas.size() + 2 * nn);
+  tris.reserve(3 * nt);
+  tri_index.reserve(3 * nt);
+  tri_mat.reserve(nt);
+  for (auto* c : {&nx, &ny, &nz}) c->reserve(nv);
   for (int m = 0; m < v->num_meshes; ++m) {
     const xb_mesh_view& mv = v->meshes[m];
     if (mv.num_triangles > 0 && (!mv.blas_nodes || mv.num_blas_nodes <= 0 || !mv.blas_prims))
@@ -2377,8 +2311,14 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
         if ((int64_t)nd.child + 1 >= mv.num_blas_nodes) return set_err(r, XB_E_INVALID, "mesh %d BLAS child out of range", m);
         child = (uint32_t)(node_base + nd.child);
       }
-      blas.push_back(node_lo(nd));
-      blas.push_back(node_hi(nd, child));
+      blas.push_back(make_float4(nd.mn[0], nd.mn[1], nd.mx[0], nd.mx[1]));
+      uint32_t entry = (nd.count << 28) | child;
+      if (nd.count >= kEntryEscape) {
+        entry = (kEntryEscape << 28) | (uint32_t)big_leaves.size();
+        big_leaves.push_back(make_uint2(child, nd.count));
+      }
+      blas.push_back(make_float4(nd.mn[2], nd.mx[2], u32_bits_to_f(entry), u32_bits_to_f(nd.count)));
+      for (int k = 0; k < 3; ++k) loose = loose || nd.mn[k] != nd.mn[k] || nd.mx[k] != nd.mx[k];
     }
     for (int s = 0; s < mv.num_triangles; ++s) {
       const uint32_t t = mv.blas_prims[s];
@@ -2431,11 +2371,10 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   }
   // ── TLAS and instances ──
   std::vector<float4> tlas;
-  for (int i = 0; i < v->num_tlas_nodes; ++i) {
-    tlas.push_back(node_lo(v->tlas_nodes[i]));
-    tlas.push_back(node_hi(v->tlas_nodes[i], v->tlas_nodes[i].child));
-  }
-  std::vector<uint32_t> tinst(v->tlas_inst_indices, v->tlas_inst_indices + v->num_instances);
+  bool loose_tlas = false;
+  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves, loose_tlas))
+    return set_err(r, XB_E_INVALID, "a TLAS node has two parents, or the TLAS is too large");
+  std::copy(tlas.begin(), tlas.end(), blas.begin());
   std::vector<DevInstance> insts(v->num_instances);
   r->inst_geom.assign(v->num_instances, 0);
   r->inst_l2w.assign(v->num_instances, xb::Affine());
@@ -2454,10 +2393,16 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
       if (v->num_prim_nodes == 0) return set_err(r, XB_E_INVALID, "instance %d uses the empty prim group", i);
     } else {
       if (iv.geom < 0 || iv.geom >= v->num_meshes) return set_err(r, XB_E_INVALID, "instance %d: bad mesh %d", i, iv.geom);
-      d.kind = 0; d.root = root_of[iv.geom]; d.mesh = iv.geom;
-      if (d.root < 0) return set_err(r, XB_E_INVALID, "instance %d uses an empty mesh", i);
+      if (root_of[iv.geom] < 0) return set_err(r, XB_E_INVALID, "instance %d uses an empty mesh", i);
+      d.kind = 0; d.mesh = iv.geom;
+      std::memcpy(&d.root, &blas[2 * (size_t)root_of[iv.geom] + 1].z, sizeof(d.root));
     }
   }
+  r->inst_dev = insts;
+  const std::vector<DevInstance> ordered =
+      in_tlas_order(insts, v->tlas_inst_indices, v->num_tlas_nodes > 0 ? v->num_instances : 0);
+  if (v->num_tlas_nodes > 0 && ordered.empty() && v->num_instances > 0)
+    return set_err(r, XB_E_INVALID, "TLAS instance index out of range");
   // ── materials, emitters, sky ──
   std::vector<DevMaterial> mats;
   bool opaque = true;
@@ -2488,15 +2433,12 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   }
   DevScene& sc = r->scene;
   std::memset(&sc, 0, sizeof(sc));
-  const float4* cp4;
-  if ((rc = dev_upload(r, blas, &sc.blas))) return rc;
+  if ((rc = dev_upload(r, blas, &sc.nodes))) return rc;
   if ((rc = dev_upload(r, tris, &sc.tris))) return rc;
+  if ((rc = dev_upload(r, big_leaves, &sc.big_leaves))) return rc;
   if ((rc = dev_upload(r, pnodes, &sc.pnodes))) return rc;
   if ((rc = dev_upload(r, prims, &sc.prims))) return rc;
-  if ((rc = dev_upload(r, tlas, &cp4))) return rc;
-  sc.tlas = cp4;
-  if ((rc = dev_upload(r, tinst, &sc.tlas_inst))) return rc;
-  if ((rc = dev_upload(r, insts, &sc.inst))) return rc;
+  if ((rc = dev_upload(r, ordered, &sc.inst))) return rc;
   if ((rc = dev_upload(r, meshes, &sc.meshes))) return rc;
   if ((rc = dev_upload(r, tri_index, &sc.tri_index))) return rc;
   if ((rc = dev_upload(r, tri_mat, &sc.tri_mat))) return rc;
@@ -2515,7 +2457,10 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.num_lights = v->num_lights;
   sc.num_suns = v->num_suns;
   sc.num_tlas_nodes = v->num_tlas_nodes;
-  r->tlas_cap = v->num_tlas_nodes;
+  if (!tlas.empty()) { sc.root_a = tlas[0]; sc.root_b = tlas[1]; }
+  r->tlas_cap = tlas_cap;
+  r->big_leaves = (int64_t)big_leaves.size();
+  r->loose_blas = loose;
   sc.num_materials = v->num_materials;
   std::memcpy(sc.sky_zenith, v->sky.zenith, sizeof(sc.sky_zenith));
   std::memcpy(sc.sky_horizon, v->sky.horizon, sizeof(sc.sky_horizon));
@@ -2523,6 +2468,7 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.sky_inv_sharpness = 1.0f / v->sky.sharpness;
   sc.sky_intensity = v->sky.intensity;
   sc.sun_nee = (r->cfg.flags & XB_FLAG_SUN_NEE) != 0;
+  sc.loose_boxes = loose || loose_tlas;
   sc.watertight = (r->cfg.flags & XB_FLAG_WATERTIGHT) != 0;
   if ((r->cfg.flags & XB_FLAG_SKY_IS) && sc.sky_intensity > 0.f) {
     std::vector<float> cdf;
@@ -2565,7 +2511,7 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   }
   char* base = static_cast<char*>(r->refit_mem);
   xb::RefitArgs a;
-  a.blas = reinterpret_cast<xb::Quad*>(const_cast<float4*>(r->scene.blas));
+  a.blas = reinterpret_cast<xb::Quad*>(const_cast<float4*>(r->scene.nodes));
   a.tris = reinterpret_cast<xb::Quad*>(const_cast<float4*>(r->scene.tris));
   a.tri_index = r->scene.tri_index;
   float* pos_dev = reinterpret_cast<float*>(base);
@@ -2575,6 +2521,9 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   a.parent = reinterpret_cast<int32_t*>(rest);
   a.arrivals = reinterpret_cast<uint32_t*>(rest + b_nodes);
   a.status = reinterpret_cast<int32_t*>(rest + 2 * b_nodes);
+  a.big_leaves = reinterpret_cast<const uint32_t*>(r->scene.big_leaves);
+  a.child_mask = kLeafEntry - 1u;
+  a.big_count = kEntryEscape;
   a.node_base = ml.node_base;
   a.slot_base = ml.slot_base;
   a.num_nodes = ml.num_nodes;
@@ -2602,7 +2551,7 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   int32_t status = 0;
   float4 root[2];
   CK(cudaMemcpyAsync(&status, a.status, sizeof(status), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(root, r->scene.blas + 2 * ml.node_base, sizeof(root), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(root, r->scene.nodes + 2 * ml.node_base, sizeof(root), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   drop_graphs(r);
   if (status != 0) {
@@ -2611,8 +2560,8 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
     return set_err(r, XB_E_INVALID, "xb_refit_mesh: mesh %d's BLAS is malformed (%s); upload the scene again",
                    mesh, status == 1 ? "an index out of range" : "a cycle");
   }
-  ml.root.mn[0] = root[0].x; ml.root.mn[1] = root[0].y; ml.root.mn[2] = root[0].z;
-  ml.root.mx[0] = root[0].w; ml.root.mx[1] = root[1].x; ml.root.mx[2] = root[1].y;
+  ml.root.mn[0] = root[0].x; ml.root.mn[1] = root[0].y; ml.root.mn[2] = root[1].x;
+  ml.root.mx[0] = root[0].z; ml.root.mx[1] = root[0].w; ml.root.mx[2] = root[1].y;
   // the TLAS over the instances' new world boxes, built on the host as xb_scene_build builds it
   std::vector<const xb_bvh_node*> roots(r->inst_geom.size(), nullptr);
   for (size_t i = 0; i < roots.size(); ++i) {
@@ -2628,22 +2577,24 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
     return set_err(r, XB_E_OOM, "xb_refit_mesh: out of host memory");
   }
   std::vector<float4> tlas;
-  for (const xb_bvh_node& n : nodes) {
-    tlas.push_back(node_lo(n));
-    tlas.push_back(node_hi(n, n.child));
-  }
+  std::vector<uint2> big((size_t)r->big_leaves);
+  bool loose_tlas = false;
   DevScene& sc = r->scene;
-  if ((int64_t)nodes.size() > r->tlas_cap) {
-    const float4* fresh;
-    if ((rc = dev_upload(r, tlas, &fresh))) return rc;
-    sc.tlas = fresh;
-    r->tlas_cap = (int64_t)nodes.size();
-  } else if (!tlas.empty()) {
-    CK(cudaMemcpy(const_cast<float4*>(sc.tlas), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice));
+  // every leaf of this TLAS is one instance, so it fits the array and adds no big leaf
+  if (!pack_tlas(nodes.data(), (int)nodes.size(), (int)r->inst_geom.size(), tlas, big, loose_tlas) ||
+      (int64_t)nodes.size() > r->tlas_cap || (int64_t)big.size() > r->big_leaves)
+    return set_err(r, XB_E_UNSUPPORTED, "xb_refit_mesh: the rebuilt TLAS does not fit the uploaded scene's");
+  if (!tlas.empty()) {
+    CK(cudaMemcpy(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    sc.root_a = tlas[0];
+    sc.root_b = tlas[1];
   }
-  if (!order.empty())
-    CK(cudaMemcpy(const_cast<uint32_t*>(sc.tlas_inst), order.data(), order.size() * sizeof(uint32_t),
+  sc.loose_boxes = r->loose_blas || loose_tlas;
+  if (!order.empty()) {
+    const std::vector<DevInstance> ordered = in_tlas_order(r->inst_dev, order.data(), order.size());
+    CK(cudaMemcpy(const_cast<DevInstance*>(sc.inst), ordered.data(), ordered.size() * sizeof(DevInstance),
                   cudaMemcpyHostToDevice));
+  }
   sc.num_tlas_nodes = (int32_t)nodes.size();
   if (!nodes.empty()) {
     for (int k = 0; k < 3; ++k) {
@@ -3047,6 +2998,12 @@ int xb_reset_profile(xb_renderer* r) {
   return XB_OK;
 }
 
+// Ray indices within a launch are 32-bit; a larger batch is several launches.
+static constexpr int64_t kMaxLaunchRays = (int64_t)1 << 30;
+static bool aligned16(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
+
 int xb_trace_rays_device(xb_renderer* r, const xb_ray* rays, int64_t n, xb_hit* hits, int32_t mode,
                          void* stream) {
   int rc = check_ready(r);
@@ -3060,14 +3017,13 @@ int xb_trace_rays_device(xb_renderer* r, const xb_ray* rays, int64_t n, xb_hit* 
   // persistent warps, each over its own contiguous range of the batch, where the renderer's
   // tuning puts its own rays of that kind on persistent warps (bounce rays for closest hits)
   const bool persistent = any ? r->tune.shadow_persistent == 1 : r->tune.extend_persistent_from_depth <= 1;
-  if (!r->thread_per_ray && persistent && n <= (int64_t)INT32_MAX / 2) {
-    const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)r->num_sms * r->occ_api[any]);
-    const int refill = std::max(1, r->tune.refill);
-    if (any) trace_api_persistent_kernel<true><<<grid, 128, 0, s>>>(r->scene, rays, (int)n, hits, r->stats, refill);
-    else trace_api_persistent_kernel<false><<<grid, 128, 0, s>>>(r->scene, rays, (int)n, hits, r->stats, refill);
-  } else {
-    const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)r->num_sms * 16);
-    trace_full_kernel<<<grid, 128, 0, s>>>(r->scene, rays, n, hits, mode, r->stats);
+  const int refill = !r->thread_per_ray && persistent ? std::max(1, r->tune.refill) : 32;
+  const bool wide = aligned16(rays, hits);
+  for (int64_t at = 0; at < n; at += kMaxLaunchRays) {
+    const int m = (int)std::min(n - at, kMaxLaunchRays);
+    const int grid = (int)std::min<int64_t>(((int64_t)m + 127) / 128, (int64_t)r->num_sms * r->occ_api[any]);
+    auto kern = any ? trace_api_persistent_kernel<true> : trace_api_persistent_kernel<false>;
+    kern<<<grid, 128, 0, s>>>(r->scene, rays + at, m, hits + at, r->stats, refill, wide);
   }
   CK(cudaGetLastError());
   return XB_OK;
@@ -3104,9 +3060,15 @@ int xb_trace_rays_noalloc(xb_renderer* r, const xb_ray* rays, int64_t n, xb_hit*
     scratch = g_noalloc_ptr[dev];
   }
   cudaStream_t s = stream ? (cudaStream_t)stream : r->stream;
-  noalloc_begin_kernel<<<1, kNoAllocScratchWords, 0, s>>>(scratch, n);
-  const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)r->num_sms * r->occ_ext);
-  trace_stealing_kernel<<<grid, 128, 0, s>>>(r->scene, rays, hits, mode, scratch, r->stats);
+  const int any = mode == XB_TRACE_ANY ? 1 : 0;
+  const bool wide = aligned16(rays, hits);
+  for (int64_t at = 0; at < n; at += kMaxLaunchRays) {
+    const int64_t m = std::min(n - at, kMaxLaunchRays);
+    noalloc_begin_kernel<<<1, kNoAllocScratchWords, 0, s>>>(scratch, m);
+    const int grid = (int)std::min<int64_t>((m + 127) / 128, (int64_t)r->num_sms * r->occ_api[any]);
+    auto kern = any ? trace_stealing_kernel<true> : trace_stealing_kernel<false>;
+    kern<<<grid, 128, 0, s>>>(r->scene, rays + at, hits + at, scratch, r->stats, std::max(1, r->tune.refill), wide);
+  }
   CK(cudaGetLastError());
   return XB_OK;
 }

@@ -463,8 +463,8 @@ void refit_blas(const HostMesh& m, std::vector<xb_bvh_node>& nodes) {
   std::vector<Quad> blas(2 * (size_t)nn), tris(3 * (size_t)nt);
   for (int32_t i = 0; i < nn; ++i) {
     const xb_bvh_node& n = nodes[i];
-    blas[2 * i] = Quad{n.mn[0], n.mn[1], n.mn[2], n.mx[0]};
-    blas[2 * i + 1] = Quad{n.mx[1], n.mx[2], bits(n.child), bits(n.count)};
+    blas[2 * i] = Quad{n.mn[0], n.mn[1], n.mx[0], n.mx[1]};
+    blas[2 * i + 1] = Quad{n.mn[2], n.mx[2], bits(n.child), bits(n.count)};
   }
   for (int32_t s = 0; s < nt; ++s) tris[3 * s].w = bits(m.prims[s]);
   std::vector<float> pos(3 * (size_t)m.num_vertices());
@@ -480,6 +480,8 @@ void refit_blas(const HostMesh& m, std::vector<xb_bvh_node>& nodes) {
   a.parent = parent.data();
   a.arrivals = arrivals.data();
   a.status = &status;
+  a.big_leaves = nullptr;
+  a.child_mask = a.big_count = 0xffffffffu;   // the entries are the children themselves
   a.node_base = 0;
   a.slot_base = 0;
   a.num_nodes = nn;
@@ -493,8 +495,8 @@ void refit_blas(const HostMesh& m, std::vector<xb_bvh_node>& nodes) {
   if (status != 0) throw std::invalid_argument("refit: malformed BLAS");
   for (int32_t i = 0; i < nn; ++i) {
     xb_bvh_node& n = nodes[i];
-    n.mn[0] = blas[2 * i].x; n.mn[1] = blas[2 * i].y; n.mn[2] = blas[2 * i].z;
-    n.mx[0] = blas[2 * i].w; n.mx[1] = blas[2 * i + 1].x; n.mx[2] = blas[2 * i + 1].y;
+    n.mn[0] = blas[2 * i].x; n.mn[1] = blas[2 * i].y; n.mn[2] = blas[2 * i + 1].x;
+    n.mx[0] = blas[2 * i].z; n.mx[1] = blas[2 * i].w; n.mx[2] = blas[2 * i + 1].y;
   }
 }
 

@@ -1,21 +1,37 @@
-// trace_persistent.cuh — persistent-warp traversal of a ray queue with per-lane refill.
+// trace_persistent.cuh — persistent-warp traversal of a ray queue with per-lane refill, the one
+// traversal of every kernel that traces rays.
 //
-// A warp holds 32 rays. Each outer iteration: lanes without a ray take new ones from the queue
-// (one atomic per warp for all idle lanes), then the warp steps its rays: in each step every
-// lane with a ray does one unit of work — a TLAS node, an instance entry, a BLAS interior node,
-// or a BLAS leaf's triangles — and a lane that finishes writes its result and becomes idle. The
-// warp leaves the step loop to refill as soon as `refill` lanes are idle, so a long ray no longer
-// holds finished lanes hostage (the one-ray-per-thread kernel averages 7-16 of 32 lanes active).
-// An earlier form deferred the leaves to a warp-wide phase after the interior work ("while-while")
-// and refilled only once every lane had a leaf pending or was done; this one was faster on every
-// workload measured (config 3 renders 13.2 -> 11.3 ms per sample; trace queries 1.3-1.8x).
+// A warp holds 32 rays, and its lanes are at one of three kinds of work: a pair of nodes (of the
+// TLAS or of a BLAS: one code), a BLAS leaf's triangles, or the way between TLAS and BLAS. Each
+// step the warp does the kind that most of its lanes wait for, for those lanes; the others wait.
+// It stays with node pairs until half of the lanes that began them have left. A lane that has
+// finished waits until `refill` lanes have, then they write their answers and take new rays
+// together. refill = 32 is one ray per thread.
 //
-// Per ray, nodes and triangles are visited in exactly the order of the reference's recursive
-// loops (tlas.cpp:172-245, blas.cpp:211-265): closest-hit results, including which of two
-// equal-t triangles wins, are the reference's. Any-hit rays (kAny) only need *whether* some
-// triangle lies in [tmin, tmax], which does not depend on order, so they descend nearest child
-// first to find occluders sooner.
+// What bounds it: issue slots and the latency of the dependent node loads (DRAM under 5 %), so the
+// aim is lanes per instruction and instructions per node. B200, one wave at a time, ms per sample
+// at 1920x1080, closest hits / any hits:
+//                                              1.31 M triangles,   261 instances of
+//                                              one instance        12 meshes
+//   each lane does whatever it is at            1.43 / 1.10         6.41 / 4.67
+//   votes, packed slab test, 256-bit loads      1.24 / 0.93         5.85 / 4.05
+//   and TLAS children tested with their parent  1.24 / 0.95         4.78 / 2.89
+// Tried and slower: voting again after every node pair (3 %), staying with node pairs down to 8
+// lanes (3 %), 64 registers for 8 blocks an SM (1-20 %), the waiting words in registers (4 %), an
+// entry distance with every BLAS entry, to drop those beyond the hit at the pop (4 %).
+//
+// Per ray, the leaves and triangles are visited in the order of the reference's recursive loops
+// (tlas.cpp:172-245, blas.cpp:211-265), so closest-hit results, including which of two equal-t
+// triangles wins, are the reference's. A BLAS child's test is the reference's, made when its parent
+// is expanded. A TLAS child is tested when its parent is expanded, too, where the reference tests
+// it when it is popped: the closest hit only comes nearer, so a child that misses then would miss
+// later; one that hits carries its entry distance on the stack, and its test at the pop is that
+// distance against the hit by then, the only term of the reference's test that has changed.
+// Any-hit rays (kAny) only need *whether* some triangle lies in [tmin, tmax], which does not depend
+// on order, so they descend nearest child first to find occluders sooner.
 #pragma once
+
+#include <type_traits>
 
 #include "dev_scene.cuh"
 
@@ -76,185 +92,252 @@ struct QueueIO {
   __device__ __forceinline__ unsigned long long* stats() const { return q.stats; }
 };
 
+// Adds a warp's traversal counters to four device totals: one atomic per warp and counter. The
+// sums of the 16-bit halves fit 32 bits.
+__device__ __forceinline__ void flush_counters(unsigned long long* dst, const TraversalCounters& c) {
+  const uint32_t v[4] = {c.nodes, c.tris, c.tlas, c.inst};
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t lo = __reduce_add_sync(0xffffffffu, v[k] & 0xffffu), hi = __reduce_add_sync(0xffffffffu, v[k] >> 16);
+    if ((threadIdx.x & 31) == 0) atomicAdd(dst + k, ((unsigned long long)hi << 16) + lo);
+  }
+}
+
 template <bool kAny, bool kCount, int kSh, class IO>
 __device__ __forceinline__ void trace_persistent(const DevScene& sc, IO& io, int refill, bool far_first) {
   constexpr unsigned FULL = 0xffffffffu;
+  using Stack = TStack<uint32_t, kSh>;
   const int lane = threadIdx.x & 31;
-  uint32_t tstack[kStackSize];
-  uint32_t bstack_local[kStackSize];
+  // a closest-hit ray's TLAS entries are two words, the entry distance below the entry
+  constexpr int kTlasWords = kAny ? 1 : 2;
+  uint32_t stack_local[(kTlasWords + 1) * kStackSize];
   extern __shared__ uint32_t s_stack[];
-  const BStack<kSh> bstack{s_stack + threadIdx.x, bstack_local};
+  const Stack stack{s_stack + threadIdx.x, stack_local};
+  // What a ray needs only between TLAS and BLAS, at a hit and at its end waits in shared memory.
+  enum { W_ORG = 0, W_DIR = 3, W_INV = 6, W_LDIR = 9, W_TMAX = 12, W_U = 13, W_V, W_PRIM, W_INST, W_WORDS };
+  __shared__ float s_ray[W_WORDS * kShStride];
+  float* const w = s_ray + threadIdx.x;
+  auto get3 = [w](int k) { return v3(w[k * kShStride], w[(k + 1) * kShStride], w[(k + 2) * kShStride]); };
+  auto put3 = [w](int k, V3 a) { w[k * kShStride] = a.x; w[(k + 1) * kShStride] = a.y; w[(k + 2) * kShStride] = a.z; };
+  auto put_hit = [w](float u, float v, int prim, int inst) {
+    w[W_U * kShStride] = u; w[W_V * kShStride] = v;
+    w[W_PRIM * kShStride] = __int_as_float(prim); w[W_INST * kShStride] = __int_as_float(inst);
+  };
   TraversalCounters cnt{0, 0, 0, 0};
   bool overflow = false;
 
   int ray = -1;                   // queue index of this lane's ray, -1 = idle
   bool exhausted = false;         // the queue has no more rays for this warp
-  V3 wo = v3s(0.f), wd = v3s(0.f), winv = v3s(0.f);
-  float tmin = 0.f, tmax = kInf;
-  int sign0 = 0, sign1 = 0, sign2 = 0;
-  V3 lo = v3s(0.f), ld = v3s(0.f), linv = v3s(0.f);
-  int tsp = 0, bsp = 0;
-  uint32_t bcur = 0;              // BLAS node being expanded (a stack entry), valid if bactive
-  bool bactive = false;
-  int cur_inst = -1;              // instance being traversed (-1: at TLAS level)
-  uint32_t tl_child = 0, tl_count = 0, tl_i = 0;   // instances of the current TLAS leaf
-  HitState h{kInf, 0.f, 0.f, -1, -1};
+  float tmin = 0.f, t_best = 0.f; // closest hits: the hit's t so far; any hits: the ray's tmax
+  SlabRay sr;                     // the ray in the space of the nodes it is among
+  sr.set(v3s(0.f), v3s(0.f));
+  bool odd = false, world_odd = false, in_blas = false;
+  int sp = 0, base = 0;           // stack entries [base, sp) belong to the BLAS (or the TLAS) it is in
+  uint32_t cur = kDone;           // the entry to expand; kNoWork: back to the TLAS; kDone: none left
+  int cur_inst = -1;
+  uint32_t tl_next = 0, tl_end = 0;   // instances left of the current TLAS leaf
   bool occluded = false;
 
-  for (;;) {
-    // ── refill idle lanes ──
-    const unsigned idle = __ballot_sync(FULL, ray < 0);
-    if (!exhausted && __popc(idle) >= refill) {
-      const int leader = __ffs(idle) - 1;
-      const int base = io.grab(lane, leader, __popc(idle));
-      if (base >= io.end()) exhausted = true;
-      if (ray < 0) {
-        const int mine = base + __popc(idle & ((1u << lane) - 1u));
-        if (mine < io.end()) {
-          ray = mine;
-          io.template load<kAny>(ray, wo, wd, tmin, tmax);
-          winv = v3(1.f / wd.x, 1.f / wd.y, 1.f / wd.z);
-          sign0 = wd.x < 0.f; sign1 = wd.y < 0.f; sign2 = wd.z < 0.f;
-          tsp = 0; bsp = 0; bactive = false; cur_inst = -1; tl_count = 0; tl_i = 0;
-          h = HitState{kInf, 0.f, 0.f, -1, -1};
-          occluded = false;
-          if (sc.num_tlas_nodes > 0) tstack[tsp++] = 0;
+  // what follows the stack's last entry: the TLAS while it holds anything
+  auto none = [&]() -> uint32_t { return in_blas && (base > 0 || tl_next != tl_end) ? kNoWork : kDone; };
+  auto pop_blas = [&]() -> uint32_t { return sp > base ? stack.get(--sp) : none(); };
+  auto pop_tlas = [&]() -> uint32_t {
+    while (sp > 0) {
+      const uint32_t e = stack.get(--sp);
+      if (kAny || __uint_as_float(stack.get(--sp)) <= t_best) return e;
+    }
+    return kDone;
+  };
+
+  // A pair of nodes (tlas.cpp:186-242, blas.cpp:222-263): the near child continues in cur, the far
+  // one is pushed. mixed: some lanes are in the TLAS (without: 5 % faster where there is one
+  // instance).
+  auto step = [&](auto mixed) {
+    const bool blas = decltype(mixed)::value ? in_blas : true;
+    if (cur < kLeafEntry) {
+      if (kCount) {
+        if (blas) cnt.nodes++;
+        else cnt.tlas += 2;
+      }
+      const float4* pp = sc.nodes + 2 * (size_t)cur;
+      float4 la, lb, ra, rb;
+      ldg8(pp, la, lb);
+      ldg8(pp + 2, ra, rb);
+      uint32_t el = __float_as_uint(lb.z), er = __float_as_uint(rb.z);
+      float tl, tr;
+      bool hl, hr;
+      if (!odd) {
+        hl = sr.slab(la, lb, tmin, t_best, tl);
+        hr = sr.slab(ra, rb, tmin, t_best, tr);
+      } else if (blas) {
+        hl = slab_sse(la, lb, sr.inv(), sr.org(), tmin, t_best, tl);
+        hr = slab_sse(ra, rb, sr.inv(), sr.org(), tmin, t_best, tr);
+      } else {
+        hl = aabb_fast(la, lb, sr.inv(), sr.org(), get3(W_DIR), tmin, t_best, tl);
+        hr = aabb_fast(ra, rb, sr.inv(), sr.org(), get3(W_DIR), tmin, t_best, tr);
+      }
+      bool left = (tl < tr) != (kAny && far_first);
+      if (!blas) {
+        if (!kAny) {
+          // the child whose centre comes first along the parent's widest axis
+          const bool ay = (el & 1u) != 0, az = (er & 1u) != 0;
+          const V3 no = sr.norg(), iv = sr.inv();
+          const float o = az ? no.z : (ay ? no.y : no.x), i = az ? iv.z : (ay ? iv.y : iv.x);
+          left = (lb.w + o) * i < (rb.w + o) * i;
         }
+        if (el < kLeafEntry) el >>= 1;
+        if (er < kLeafEntry) er >>= 1;
+      }
+      if (hl && hr) {
+        if (sp - base >= (blas ? kStackSize : kTlasWords * (kStackSize - 1))) {
+          overflow = true;
+          cur = kDone;            // abandon (reported as overflow)
+        } else {
+          const uint32_t far = left ? er : el;
+          if (!kAny && !blas) stack.put(sp++, __float_as_uint(left ? tr : tl));
+          stack.put(sp++, far);
+          cur = left ? el : er;
+        }
+      } else if (hl || hr) {
+        cur = hl ? el : er;
+      } else {
+        cur = blas ? pop_blas() : pop_tlas();
       }
     }
-    if (__ballot_sync(FULL, ray >= 0) == 0 && exhausted) break;
+  };
 
-    // ── steps until enough lanes are idle to refill (or, the queue exhausted, all are) ──
-    bool want = (ray >= 0);
-    while (__any_sync(FULL, want)) {
-      if (want) {
-        if (bactive) {
-          // BLAS node (blas.cpp:222-263): the near child continues in bcur, the far one is pushed
-          uint32_t child, count;
-          blas_unpack(sc, bcur, child, count);
-          if (count > 0) {
-            // the leaf's triangles (blas.cpp:224-233 / 281-287)
-            float tbest = kAny ? tmax : h.t;
-            for (uint32_t i = 0; i < count; ++i) {
-              const float4* tp = sc.tris + 3 * (size_t)(child + i);
-              const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
-              if (kCount) cnt.tris++;
-              float t, u, v;
-              if (tri_hit(sc, lo, ld, linv, tmin, ld3(a), ld3(b), ld3(c), kAny ? tmax : tbest, t, u, v)) {
-                if (kAny) {
-                  occluded = true;
-                  break;
-                }
-                tbest = t;
-                h.t = t; h.u = u; h.v = v;
-                h.prim = (int32_t)(child + i);
-                h.inst = cur_inst;
-              }
-            }
-            if (kAny && occluded) {
-              bsp = 0; tsp = 0; tl_count = 0; bactive = false;
-            } else if (bsp > 0) {
-              bcur = bstack.get(--bsp);
-            } else {
-              bactive = false;
-            }
-          } else {
-            if (kCount) cnt.nodes++;
-            const float4* pp = sc.blas + 2 * (size_t)child;
-            const float4 la = ldg4(pp), lb = ldg4(pp + 1), ra = ldg4(pp + 2), rb = ldg4(pp + 3);
-            float tl, tr;
-            const float tcull = kAny ? tmax : h.t;
-            const bool hl = slab_sse(la, lb, linv, lo, tmin, tcull, tl);
-            const bool hr = slab_sse(ra, rb, linv, lo, tmin, tcull, tr);
-            const uint32_t el = blas_entry(__float_as_uint(lb.z), __float_as_uint(lb.w), child);
-            const uint32_t er = blas_entry(__float_as_uint(rb.z), __float_as_uint(rb.w), child + 1);
-            if (hl && hr) {
-              if (bsp + 1 > kStackSize) {
-                overflow = true;
-                bactive = false; bsp = 0; tsp = 0; tl_count = 0;   // abandon (reported as overflow)
-              } else if ((tl < tr) != (kAny && far_first)) {
-                bstack.put(bsp++, er); bcur = el;
-              } else {
-                bstack.put(bsp++, el); bcur = er;
-              }
-            } else if (hl || hr) {
-              bcur = hl ? el : er;
-            } else if (bsp > 0) {
-              bcur = bstack.get(--bsp);
-            } else {
-              bactive = false;
+  for (;;) {
+    // ── write finished rays' answers and take new ones, several lanes at once ──
+    unsigned idle = __ballot_sync(FULL, cur == kDone);
+    bool to_top = false;
+    if (idle == FULL || (!exhausted && __popc(idle) >= refill)) {
+      if (cur == kDone && ray >= 0) {
+        if (kAny) io.finish_any(ray, occluded);
+        else io.finish_closest(sc, ray, get3(W_ORG), get3(W_DIR), tmin, w[W_TMAX * kShStride],
+                               HitState{t_best, w[W_U * kShStride], w[W_V * kShStride],
+                                        __float_as_int(w[W_PRIM * kShStride]), __float_as_int(w[W_INST * kShStride])});
+        ray = -1;
+      }
+      if (exhausted) break;
+      const int first = io.grab(lane, __ffs(idle) - 1, __popc(idle));
+      if (first >= io.end()) exhausted = true;
+      if (cur == kDone) {
+        const int mine = first + __popc(idle & ((1u << lane) - 1u));
+        if (mine < io.end()) {
+          ray = mine;
+          V3 wo, wd;
+          float tmax;
+          io.template load<kAny>(ray, wo, wd, tmin, tmax);
+          const V3 winv = v3(1.f / wd.x, 1.f / wd.y, 1.f / wd.z);
+          put3(W_ORG, wo);
+          put3(W_DIR, wd);
+          put3(W_INV, winv);
+          w[W_TMAX * kShStride] = tmax;
+          t_best = kAny ? tmax : kInf;
+          if (!kAny) put_hit(0.f, 0.f, -1, -1);
+          sr.set(wo, winv);
+          odd = world_odd = SlabRay::odd(sc, wo, winv, tmin, t_best);
+          sp = 0; base = 0; tl_next = 0; tl_end = 0;
+          in_blas = false;
+          occluded = false;
+          if (sc.num_tlas_nodes > 0) {
+            if (kCount) cnt.tlas++;
+            float tn;
+            if (odd ? aabb_fast(sc.root_a, sc.root_b, winv, wo, wd, tmin, t_best, tn)
+                    : sr.slab(sc.root_a, sc.root_b, tmin, t_best, tn)) {
+              cur = __float_as_uint(sc.root_b.z);
+              if (cur < kLeafEntry) cur >>= 1;
             }
           }
-        } else if (tl_i < tl_count) {
-          // enter the next instance of the current TLAS leaf (tlas.cpp:200-218)
-          const int ii = (int)__ldg(sc.tlas_inst + tl_child + tl_i);
-          ++tl_i;
-          const DevInstance& in = sc.inst[ii];
-          if (kCount) cnt.inst++;
-          const Ray wr{wo, wd, tmin, tmax};
-          const Ray lr = to_local(in, wr);
-          if (in.kind == 0) {
-            lo = lr.o; ld = lr.d;
-            linv = v3(1.f / ld.x, 1.f / ld.y, 1.f / ld.z);
-            cur_inst = ii;
-            bcur = blas_root_entry(sc, in.root);
-            bactive = true;
-          } else {
-            // analytic prims: a short scalar walk, done in place
-            if (kAny) {
-              if (pblas_any(sc, lr, bstack, overflow)) { occluded = true; bsp = 0; bactive = false; tsp = 0; tl_count = 0; }
-            } else {
-              pblas_closest(sc, lr, h, ii, bstack, overflow);
-            }
-          }
-          if (kAny && occluded) want = false;
-        } else if (tsp > 0) {
-          // TLAS node (tlas.cpp:186-242)
-          const uint32_t idx = tstack[--tsp];
-          const float4 na = ldg4(sc.tlas + 2 * idx), nb = ldg4(sc.tlas + 2 * idx + 1);
-          if (kCount) cnt.tlas++;
-          const int sgn[3] = {sign0, sign1, sign2};
-          if (aabb_fast(na, nb, winv, wo, sgn, tmin, kAny ? tmax : h.t)) {
-            const uint32_t child = __float_as_uint(nb.z), count = __float_as_uint(nb.w);
-            if (count > 0) {
-              tl_child = child; tl_count = count; tl_i = 0;
-            } else if (tsp + 2 > kStackSize) {
-              overflow = true;
-              tsp = 0;
-            } else {
-              const float ex = na.w - na.x, ey = nb.x - na.y, ez = nb.y - na.z;
-              const int ax = (ex > ey && ex > ez) ? 0 : (ey > ez ? 1 : 2);
-              const float4 la = ldg4(sc.tlas + 2 * child), lb = ldg4(sc.tlas + 2 * child + 1);
-              const float4 ra = ldg4(sc.tlas + 2 * child + 2), rb = ldg4(sc.tlas + 2 * child + 3);
-              float cl, cr;
-              if (ax == 0) { cl = (la.x + la.w) * 0.5f; cr = (ra.x + ra.w) * 0.5f; }
-              else if (ax == 1) { cl = (la.y + lb.x) * 0.5f; cr = (ra.y + rb.x) * 0.5f; }
-              else { cl = (la.z + lb.y) * 0.5f; cr = (ra.z + rb.y) * 0.5f; }
-              const float tl = (cl - comp(wo, ax)) * comp(winv, ax);
-              const float tr = (cr - comp(wo, ax)) * comp(winv, ax);
-              if (tl < tr) { tstack[tsp++] = child + 1; tstack[tsp++] = child; }
-              else { tstack[tsp++] = child; tstack[tsp++] = child + 1; }
-            }
-          }
-        } else {
-          // ray finished
-          want = false;
-          if (kAny) io.finish_any(ray, occluded);
-          else io.finish_closest(sc, ray, wo, wd, tmin, tmax, h);
-          ray = -1;
         }
       }
-      if (!exhausted && __popc(__ballot_sync(FULL, ray < 0)) >= refill) break;
+      // then the way into an instance, for new rays whose TLAS is one leaf, while they are together
+      idle = __ballot_sync(FULL, cur == kDone);
+      to_top = true;
+    }
+    // ── one kind of work for the lanes that are at it: the kind most lanes wait for ──
+    const int n_inner = __popc(__ballot_sync(FULL, cur < kLeafEntry));
+    const int n_leaf = __popc(__ballot_sync(FULL, in_blas && cur >= kLeafEntry && cur < kDone));
+    const int n_top = 32 - n_inner - n_leaf - __popc(idle);
+    if (!to_top && n_inner >= n_leaf && n_inner >= n_top) {
+      const int keep = max(1, (n_inner + 1) / 2);
+      if (__any_sync(FULL, cur < kLeafEntry && !in_blas)) {
+        do step(std::true_type{}); while (__popc(__ballot_sync(FULL, cur < kLeafEntry)) >= keep);
+      } else {
+        do step(std::false_type{}); while (__popc(__ballot_sync(FULL, cur < kLeafEntry)) >= keep);
+      }
+    } else if (!to_top && n_leaf >= n_top) {
+      if (in_blas && cur >= kLeafEntry && cur < kDone) {
+        // the leaf's triangles (blas.cpp:224-233 / 281-287)
+        uint32_t first, count;
+        leaf_unpack(sc, cur, first, count);
+        const V3 lo = sr.org(), linv = sr.inv(), ld = get3(W_LDIR);
+        for (uint32_t i = 0; i < count; ++i) {
+          const float4* tp = sc.tris + 3 * (size_t)(first + i);
+          const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
+          if (kCount) cnt.tris++;
+          float t, u, v;
+          if (tri_hit(sc, lo, ld, linv, tmin, ld3(a), ld3(b), ld3(c), t_best, t, u, v)) {
+            if (kAny) {
+              occluded = true;
+              break;
+            }
+            t_best = t;
+            put_hit(u, v, (int)(first + i), cur_inst);
+          }
+        }
+        cur = kAny && occluded ? kDone : pop_blas();
+      }
+    } else if (cur >= kLeafEntry && cur != kDone && (!in_blas || cur == kNoWork)) {
+      if (cur == kNoWork && tl_next == tl_end) {
+        // back among the TLAS nodes
+        in_blas = false;
+        base = 0;
+        odd = world_odd;
+        sr.set(get3(W_ORG), get3(W_INV));
+        cur = pop_tlas();
+      }
+      if (cur >= kLeafEntry && cur < kDone) {
+        uint32_t first, count;
+        leaf_unpack(sc, cur, first, count, 1);
+        tl_next = first;
+        tl_end = first + count;
+        cur = kNoWork;
+      }
+      if (cur == kNoWork && tl_next != tl_end) {
+        // enter the next instance of the current TLAS leaf (tlas.cpp:200-218)
+        const int ii = (int)tl_next++;
+        const DevInstance in = load_instance(sc.inst + ii);
+        if (kCount) cnt.inst++;
+        const Ray lr = to_local(in, Ray{get3(W_ORG), get3(W_DIR), tmin, w[W_TMAX * kShStride]});
+        if (in.kind == 0) {
+          const V3 linv = v3(1.f / lr.d.x, 1.f / lr.d.y, 1.f / lr.d.z);
+          put3(W_LDIR, lr.d);
+          sr.set(lr.o, linv);
+          odd = SlabRay::odd(sc, lr.o, linv, tmin, t_best);
+          in_blas = true;
+          base = sp;
+          cur_inst = ii;
+          cur = in.root;
+        } else {
+          // analytic prims: a short scalar walk, done in place
+          const StackAbove<Stack> above{stack, sp};
+          if (kAny) {
+            if (pblas_any(sc, lr, above, overflow)) { occluded = true; cur = kDone; }
+          } else {
+            HitState h{t_best, 0.f, 0.f, -1, -1};
+            if (pblas_closest(sc, lr, h, ii, above, overflow)) {
+              t_best = h.t;
+              put_hit(h.u, h.v, h.prim, h.inst);
+            }
+          }
+        }
+      }
     }
   }
   if (overflow) atomicAdd(io.stats() + 3, 1ull);
-  if (kCount) {
-    unsigned long long* dst = io.stats() + (kAny ? 12 : 8);
-    atomicAdd(dst + 0, (unsigned long long)cnt.nodes);
-    atomicAdd(dst + 1, (unsigned long long)cnt.tris);
-    atomicAdd(dst + 2, (unsigned long long)cnt.tlas);
-    atomicAdd(dst + 3, (unsigned long long)cnt.inst);
-  }
+  if (kCount) flush_counters(io.stats() + (kAny ? 12 : 8), cnt);
 }
 
 }  // namespace xbd
