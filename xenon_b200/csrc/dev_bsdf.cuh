@@ -168,6 +168,26 @@ __device__ __forceinline__ float mfr_pdf(V3 wo, V3 wi, const DevMaterial& m) {
   float jac = 1.f / (4.f * fabsf(dot(wo, wh)));
   return dv * jac;
 }
+// mfr_eval and mfr_pdf of one pair of directions: the same operations, the half vector, the
+// distribution and Lambda(wo) computed once.
+__device__ __forceinline__ void mfr_eval_pdf(V3 wo, V3 wi, const DevMaterial& m, V3& f, float& pdf) {
+  f = v3s(0.f);
+  pdf = 0.f;
+  if (wo.z <= 0.f || wi.z <= 0.f) return;
+  const V3 wh = normalize(wo + wi);
+  if (wh.z <= 0.f) return;
+  const float d = ggx_d_aniso(wh, m.alpha_x, m.alpha_y);
+  const float lo = ggx_lambda_aniso(wo, m.alpha_x, m.alpha_y), li = ggx_lambda_aniso(wi, m.alpha_x, m.alpha_y);
+  const float dwo = dot(wo, wh);
+  const float denom = 4.f * wo.z * wi.z;
+  if (!(denom < 1e-8f)) {
+    f = mf_fresnel(dwo, m) * d * (1.f / (1.f + lo + li)) / denom;
+    if (!(m.flags & kMatTransmissive)) f = f * multiscatter(m, wo.z, wi.z);
+  }
+  const float co = fabsf(wo.z);
+  const float dv = co < 1e-8f ? 0.f : d * (1.f / (1.f + lo)) * smax(0.f, dwo) / co;
+  pdf = dv * (1.f / (4.f * fabsf(dwo)));
+}
 __device__ __forceinline__ bool mfr_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample& s) {
   if (wo.z <= 0.f) return false;
   // The reference passes rng.next_float() twice as call arguments; GCC evaluates them right
@@ -218,6 +238,31 @@ __device__ __forceinline__ float mft_pdf(V3 wo, V3 wi, const DevMaterial& m) {
   if (fabsf(denom) < 1e-8f) return 0.f;
   float dwh = fabsf((eta * eta * dwi) / (denom * denom));
   return pwh * dwh;
+}
+// mft_eval and mft_pdf of one pair of directions, as mfr_eval_pdf.
+__device__ __forceinline__ void mft_eval_pdf(V3 wo, V3 wi, const DevMaterial& m, V3& fv, float& pdf) {
+  fv = v3s(0.f);
+  pdf = 0.f;
+  if (wo.z == 0.f || wi.z == 0.f) return;
+  if (same_hemisphere(wo, wi)) return;
+  const float eta = (wo.z > 0.f) ? (1.f / m.ior) : m.ior;
+  V3 wh = normalize(wo + eta * wi);
+  if (wh.z < 0.f) wh = -wh;
+  const float dwo = dot(wo, wh), dwi = dot(wi, wh);
+  if (dwo * dwi >= 0.f) return;
+  const float d = ggx_d_aniso(wh, m.alpha_x, m.alpha_y);
+  const float lo = ggx_lambda_aniso(wo, m.alpha_x, m.alpha_y), li = ggx_lambda_aniso(wi, m.alpha_x, m.alpha_y);
+  const float co = fabsf(wo.z), ci = fabsf(wi.z);
+  const float denom = dwo + eta * dwi;
+  const float denom2 = denom * denom;
+  if (fabsf(denom) < 1e-8f) return;
+  if (!(co < 1e-8f || ci < 1e-8f)) {
+    const float f = fresnel_dielectric(dwo, m.ior);
+    const float factor = fabsf(dwo * dwi) * (eta * eta) / (co * ci * denom2);
+    fv = mat_base(m) * ((1.f - f) * d * (1.f / (1.f + lo + li)) * factor);
+  }
+  const float dv = co < 1e-8f ? 0.f : d * (1.f / (1.f + lo)) * smax(0.f, dwo) / co;
+  pdf = dv * fabsf((eta * eta * dwi) / denom2);
 }
 __device__ __forceinline__ bool mft_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample& s) {
   if (fabsf(wo.z) < 1e-8f) return false;
@@ -392,6 +437,106 @@ XB_BSDF_ENTRY bool bsdf_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample
   if (!cosine_sample(wo, mat_base(m), m, rng, s)) return false;
   s.pdf *= diff;
   return true;
+}
+
+// ── the bounce kernels' forms: bsdf_eval, bsdf_pdf and bsdf_sample around one evaluation ──
+// A bounce evaluates the microfacet lobes up to three times: for the area light, for the sun and
+// for the direction it samples. Inlined at each place (and once per material kind) they made a
+// kernel of 287 KB of code whose warps waited 43 to 79 cycles per instruction for the instruction
+// cache; the kernels therefore loop over the three with one copy of the evaluation between the
+// lobe choice (before) and the combination (after).
+enum { kLobeNone = 0, kLobeMfr = 1, kLobeMft = 2 };
+
+// The lobe that next-event estimation evaluates (wi.z > 0, not a delta material).
+template <bool kOpaque>
+__device__ __forceinline__ int nee_lobe(const DevMaterial& m) {
+  const uint32_t fl = lobe_flags<kOpaque>(m);
+  return (fl & kMatSubsurface) && !(fl & (kMatConductor | kMatTransmissive)) ? kLobeNone : kLobeMfr;
+}
+// bsdf_eval and bsdf_pdf for wi.z > 0 from the lobe's f and pdf; fo: fresnel_dielectric(|wo.z|) of a
+// transmissive material.
+template <bool kOpaque>
+__device__ __forceinline__ void nee_combine(V3 wi, const DevMaterial& m, float fo, V3& f, float& pdf) {
+  const uint32_t fl = lobe_flags<kOpaque>(m);
+  if (fl & kMatConductor) return;
+  if (fl & kMatTransmissive) {
+    pdf = fo * pdf;
+    return;
+  }
+  if (fl & kMatSubsurface) {
+    f = ss_color(m) * (1.f - m.metallic) * kInvPi;
+    pdf = diffuse_pdf(wi);
+    return;
+  }
+  const float spec = m.f0[0];
+  const float diff = 1.f - spec;
+  f = diffuse_eval(wi, m) * diff + f * spec;
+  pdf = diffuse_pdf(wi) * diff + pdf * spec;
+}
+
+// bsdf_sample up to the evaluation: the lobe, its direction and the factor of its pdf. With lobe
+// kLobeNone s is complete but for that factor. False where bsdf_sample fails before it evaluates.
+template <bool kOpaque>
+__device__ __forceinline__ bool sample_direction(V3 wo, const DevMaterial& m, float fo, Pcg& rng, BsdfSample& s,
+                                                 int& lobe, float& scale) {
+  s.delta = false;
+  s.pdf = 0.f;
+  s.f = v3s(0.f);
+  s.wi = v3s(0.f);
+  lobe = kLobeMfr;
+  scale = 1.f;
+  const uint32_t fl = lobe_flags<kOpaque>(m);
+  if (fl & kMatDelta) {
+    lobe = kLobeNone;
+    if ((fl & kMatTransmissive) && !(rng.next_float() < fo)) return delta_trans_sample(wo, m, s);
+    return delta_refl_sample(wo, m, s);
+  }
+  if (fl & kMatConductor) {
+  } else if (fl & kMatSubsurface) {
+    lobe = kLobeNone;
+  } else if (fl & kMatTransmissive) {
+    if (rng.next_float() < fo) {
+      scale = fo;
+    } else {
+      lobe = kLobeMft;
+      scale = 1.f - fo;
+    }
+  } else {
+    const float spec = sclamp(m.f0[0], 0.f, 1.f);
+    scale = spec;
+    if (!(rng.next_float() < spec)) {
+      lobe = kLobeNone;
+      scale = 1.f - spec;
+    }
+  }
+  if (lobe == kLobeMfr ? wo.z <= 0.f : (lobe == kLobeMft && fabsf(wo.z) < 1e-8f)) return false;
+  // every lobe draws u2, then u1 (see mfr_sample)
+  const float u2 = rng.next_float();
+  const float u1 = rng.next_float();
+  if (lobe == kLobeNone) {
+    s.wi = sample_cosine_hemisphere(u1, u2);
+    if (wo.z < 0.f) s.wi.z = -s.wi.z;
+    s.pdf = fabsf(s.wi.z) * kInvPi;
+    if (s.pdf < 1e-8f) return false;
+    s.f = ((fl & kMatSubsurface) ? ss_color(m) : mat_base(m)) * (1.f - m.metallic) * kInvPi;
+    return true;
+  }
+  V3 wh = sample_vndf(wo, m.alpha_x, m.alpha_y, u1, u2);
+  if (lobe == kLobeMfr) {
+    if (wh.z <= 0.f) return false;
+    s.wi = reflect(-wo, wh);
+    return !(s.wi.z <= 0.f);
+  }
+  if (wh.z < 0.f) wh = -wh;
+  const float eta = (wo.z > 0.f) ? (1.f / m.ior) : m.ior;
+  const float dwo = dot(wo, wh);
+  const float s2o = smax(0.f, 1.f - dwo * dwo);
+  const float s2i = eta * eta * s2o;
+  if (s2i >= 1.f) return false;
+  const float cti = sqrtf(smax(0.f, 1.f - s2i));
+  const float sg = (dwo > 0.f) ? 1.f : -1.f;
+  s.wi = normalize((-eta * wo) + (eta * dwo - sg * cti) * wh);
+  return !same_hemisphere(wo, s.wi);
 }
 
 // ── the sampler's true densities (guided sampling; no reference counterpart) ──────

@@ -341,11 +341,91 @@ __device__ __forceinline__ void add_L(float4* L, int p, V3 c) {
   L[p] = l;
 }
 
+// Emitter hit + MIS (cpu_tiled.cpp:62-86): the light that the hit is on adds its emission. True
+// when it is on one.
+__device__ __forceinline__ bool emitter_hit(const ShadeArgs& a, const FullHit& fh, V3 wo, float t, V3 tp,
+                                            float prev_pdf, int32_t pid) {
+  const DevScene& sc = a.sc;
+  for (int li = 0; li < sc.num_lights; ++li) {
+    const DevLight& lt = sc.lights[li];
+    if (__float_as_int(lt.p2.w) == fh.prim_id && __float_as_int(lt.p1.w) == fh.instance_id) {
+      float mis = 1.0f;
+      const float cos_l = smax(0.0f, dot(fh.geo_normal, wo));
+      if (cos_l > 1e-6f) {
+        if (a.depth > 0 && !(prev_pdf < 0.f)) {   // < 0: the previous bounce was delta
+          const float pdf_area = (1.0f / lt.p0.w) * (1.0f / (float)sc.num_lights);
+          const float dsq = t * t;
+          const float pdf_sa = (pdf_area * dsq) / cos_l;
+          mis = mis_power2(prev_pdf, pdf_sa);
+        }
+        add_L(a.L, pid, tp * v3(lt.emission.x, lt.emission.y, lt.emission.z) * mis);
+      }
+      return true;
+    }
+  }
+  return false;
+}
+
+// What next-event estimation connects to: direction, emission, density (per steradian), and the
+// shadow ray's length. The draws are the reference's.
+struct NeeLight {
+  V3 wi, emission;
+  float pdf, tmax;
+};
+// cpu_tiled.cpp:89-127
+__device__ __forceinline__ bool area_light(const DevScene& sc, V3 pos, Pcg& rng, NeeLight& nl) {
+  const float upick = rng.next_float();
+  int li = (int)(upick * (float)sc.num_lights);
+  li = li < 0 ? 0 : (li > sc.num_lights - 1 ? sc.num_lights - 1 : li);
+  const float pick_pdf = 1.f / (float)sc.num_lights;
+  const DevLight& lt = sc.lights[li];
+  const float u1 = rng.next_float();
+  const float u2 = rng.next_float();
+  const float su1 = sqrtf(u1);
+  const float b0 = 1.0f - su1;
+  const float b1 = u2 * su1;
+  const float b2 = 1.0f - b0 - b1;
+  const V3 lp = ld3(lt.p0) * b0 + ld3(lt.p1) * b1 + ld3(lt.p2) * b2;
+  const V3 ln = ld3(lt.n);
+  const V3 sdir = lp - pos;
+  const float dsq = length_sq(sdir);
+  const float dist = sqrtf(dsq);
+  if (!(dist > 1e-6f)) return false;
+  nl.wi = sdir / dist;
+  const float cos_l = smax(0.0f, dot(ln, -nl.wi));
+  if (!(cos_l > 1e-6f)) return false;
+  nl.emission = v3(lt.emission.x, lt.emission.y, lt.emission.z);
+  nl.pdf = ((1.0f / lt.p0.w) * pick_pdf) * (dsq / cos_l);
+  nl.tmax = dist - kShadowEps;
+  return true;
+}
+// cpu_tiled.cpp:148-165
+__device__ __forceinline__ bool sun_light(const DevScene& sc, Pcg& rng, NeeLight& nl) {
+  const float upick = rng.next_float();
+  int di = (int)(upick * (float)sc.num_suns);
+  di = di < 0 ? 0 : (di > sc.num_suns - 1 ? sc.num_suns - 1 : di);
+  const float dpick = 1.f / (float)sc.num_suns;
+  if (!(dpick > 0.f)) return false;
+  const DevSun& sun = sc.suns[di];
+  nl.wi = v3(sun.dir[0], sun.dir[1], sun.dir[2]);
+  nl.emission = v3(sun.emission[0], sun.emission[1], sun.emission[2]);
+  nl.pdf = sc.sun_nee ? dpick : 1e8f * dpick;
+  nl.tmax = kInf;
+  return true;
+}
+enum { PASS_AREA = 0, PASS_SUN = 1, PASS_NEXT = 2 };
+
 // kOcc: the blocks of 128 threads the kernel is compiled to fit on one SM (xb_tuning
-// shade_occupancy): 4 keeps every value in registers (108), 8, 12 and 16 cap them at 64, 40 and
-// 32 and spill the rest to L1; the bounce is latency-bound, so more resident warps usually win.
-// kOpaque: the form for scenes without delta, transmissive or subsurface materials (smaller
-// code: the bounce's largest stall is the instruction cache), the same results.
+// shade_occupancy): 4 keeps every value in registers (96-104), 8, 12 and 16 cap them at 64, 40 and
+// 32 and spill the rest to L1.
+// kOpaque: the form for scenes without delta, transmissive or subsurface materials, the same
+// results.
+// What bounds it: the dependent loads of the hit's triangle, normals and material, and lanes whose
+// path has ended. It was the instruction cache (see the bounce kernels' forms in dev_bsdf.cuh).
+// B200, ms per sample at 1920x1080, before and after the passes around one evaluation, at kOcc 4 /
+// 8 / 12 / 16: 261 instances of every material kind (287 -> 84 KB of code) 4.75 / 3.80 / 3.21 / 2.89
+// -> 1.06 / 1.15 / 1.23 / 1.33; one opaque mesh (170 -> 62 KB) 1.01 / 0.79 / 0.74 / 0.70 -> 0.54 /
+// 0.47 / 0.51 / 0.62.
 template <int kOcc, bool kOpaque>
 __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
   const int n = a.cnt[CNT_RAYS];
@@ -353,161 +433,114 @@ __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
   const bool last_all = (a.depth + 1 >= a.max_bounces);
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int slot = base + threadIdx.x;
-    bool emit_next = false, emit_area = false, emit_sun = false;
-    float4 n_o, n_d, n_tp;
-    uint64_t n_rng = 0;
+    // ── the hit: sky, emitter + MIS, or a vertex to shade ──
+    bool alive = false, last = last_all;
     int32_t pid = 0;
-    float4 a_o, a_d, a_c, s_o, s_d, s_c;
+    V3 tp = v3s(0.f), wo = v3s(0.f);
+    Pcg rng{0};
+    FullHit fh;
+    fh.mat_id = 0;
     if (slot < n) {
       const float4 ro = a.ray_o[slot], rd = a.ray_d[slot], tpv = a.tp[slot];
       pid = a.path[slot];
-      const bool last = a.path_maxd ? (a.depth + 1 >= (int)a.path_maxd[pid]) : last_all;
-      Pcg rng{a.rng[slot]};
+      if (a.path_maxd) last = a.depth + 1 >= (int)a.path_maxd[pid];
+      rng.state = a.rng[slot];
       const Ray ray{v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z), ro.w, rd.w};
-      V3 tp = v3(tpv.x, tpv.y, tpv.z);
-      const float prev_pdf = tpv.w;             // < 0: previous bounce was delta
+      tp = v3(tpv.x, tpv.y, tpv.z);
+      wo = -ray.d;
       const float4 hv = a.hit[slot];
       const int hinst = a.hit_inst[slot];
-      do {
-        if (hinst < 0) {
-          if (sc.sky_intensity > 0.f) add_L(a.L, pid, tp * sky_eval(sc, ray.d));
-          break;
-        }
-        HitState h{hv.x, hv.y, hv.z, __float_as_int(hv.w), hinst};
-        FullHit fh;
+      if (hinst < 0) {
+        if (sc.sky_intensity > 0.f) add_L(a.L, pid, tp * sky_eval(sc, ray.d));
+      } else {
+        const HitState h{hv.x, hv.y, hv.z, __float_as_int(hv.w), hinst};
         complete_hit(sc, ray, h, fh);
+        alive = !emitter_hit(a, fh, wo, h.t, tp, tpv.w, pid);
+      }
+    }
+    // ── area-light and directional-light NEE (cpu_tiled.cpp:89-187), roulette and the next
+    // direction (:190-216): one pass each around one copy of the BSDF's evaluation ──
+#pragma unroll 1
+    for (int pass = PASS_AREA; pass <= PASS_NEXT; ++pass) {
+      if (pass == PASS_AREA && sc.num_lights == 0) continue;
+      if (pass == PASS_SUN && sc.num_suns == 0) continue;
+      if (pass == PASS_NEXT && last_all) break;   // the reference samples once more, unused
+      bool emit = false;
+      float4 q_o, q_d, q_c;
+      if (alive) do {
         const DevMaterial& mat = sc.mats[fh.mat_id];
-        // ── emitter hit + MIS (cpu_tiled.cpp:62-86) ──
-        bool hit_light = false;
-        for (int li = 0; li < sc.num_lights; ++li) {
-          const DevLight& lt = sc.lights[li];
-          if (__float_as_int(lt.p2.w) == fh.prim_id && __float_as_int(lt.p1.w) == fh.instance_id) {
-            float mis = 1.0f;
-            const float cos_l = smax(0.0f, dot(fh.geo_normal, -ray.d));
-            if (cos_l > 1e-6f) {
-              if (a.depth > 0 && !(prev_pdf < 0.f)) {
-                const float pdf_area = (1.0f / lt.p0.w) * (1.0f / (float)sc.num_lights);
-                const float dsq = h.t * h.t;
-                const float pdf_sa = (pdf_area * dsq) / cos_l;
-                mis = mis_power2(prev_pdf, pdf_sa);
-              }
-              add_L(a.L, pid, tp * v3(lt.emission.x, lt.emission.y, lt.emission.z) * mis);
-            }
-            hit_light = true;
-            break;
-          }
-        }
-        if (hit_light) break;
-        const bool is_delta = (mat.flags & kMatDelta) != 0;
-        // ── area-light NEE (cpu_tiled.cpp:89-139) ──
-        if (sc.num_lights > 0 && !is_delta) {
-          const float upick = rng.next_float();
-          int li = (int)(upick * (float)sc.num_lights);
-          li = li < 0 ? 0 : (li > sc.num_lights - 1 ? sc.num_lights - 1 : li);
-          const float pick_pdf = 1.f / (float)sc.num_lights;
-          const DevLight& lt = sc.lights[li];
-          const float u1 = rng.next_float();
-          const float u2 = rng.next_float();
-          const float su1 = sqrtf(u1);
-          const float b0 = 1.0f - su1;
-          const float b1 = u2 * su1;
-          const float b2 = 1.0f - b0 - b1;
-          const V3 lp = ld3(lt.p0) * b0 + ld3(lt.p1) * b1 + ld3(lt.p2) * b2;
-          const V3 ln = ld3(lt.n);
-          const V3 sdir = lp - fh.pos;
-          const float dsq = length_sq(sdir);
-          const float dist = sqrtf(dsq);
-          if (dist > 1e-6f) {
-            const V3 wi = sdir / dist;
-            const float cos_l = smax(0.0f, dot(ln, -wi));
-            const Onb onb(fh.geo_normal);
-            const V3 wo_l = onb.to_local(-ray.d);
-            const V3 wi_l = onb.to_local(wi);
-            if (cos_l > 1e-6f && wi_l.z > 1e-6f) {
-              const V3 f = bsdf_eval<kOpaque>(wo_l, wi_l, mat);
-              const float bp = bsdf_pdf<kOpaque>(wo_l, wi_l, mat);
-              const float lpdf = ((1.0f / lt.p0.w) * pick_pdf) * (dsq / cos_l);
-              const float mis = mis_power2(lpdf, bp);
-              const float cs = wi_l.z;
-              if (mis > 0.0f && lpdf > 1e-12f) {
-                const V3 org = offset_origin(fh.pos, fh.geo_normal, wi, kShadowEps);
-                const V3 c = tp * f * cs * (v3(lt.emission.x, lt.emission.y, lt.emission.z) / lpdf) * mis;
-                a_o = make_float4(org.x, org.y, org.z, dist - kShadowEps);
-                a_d = make_float4(wi.x, wi.y, wi.z, __int_as_float(pid));
-                a_c = make_float4(c.x, c.y, c.z, 0.f);
-                emit_area = true;
-              }
-            }
-          }
-        }
-        // ── directional-light NEE (cpu_tiled.cpp:148-187) ──
-        if (sc.num_suns > 0 && !is_delta) {
-          const float upick = rng.next_float();
-          int di = (int)(upick * (float)sc.num_suns);
-          di = di < 0 ? 0 : (di > sc.num_suns - 1 ? sc.num_suns - 1 : di);
-          const float dpick = 1.f / (float)sc.num_suns;
-          if (dpick > 0.f) {
-            const DevSun& sun = sc.suns[di];
-            const V3 sdir = v3(sun.dir[0], sun.dir[1], sun.dir[2]);
-            const Onb onb(fh.geo_normal);
-            const V3 wo_l = onb.to_local(-ray.d);
-            const V3 wi_l = onb.to_local(sdir);
-            if (wi_l.z > 1e-6f) {
-              const V3 f = bsdf_eval<kOpaque>(wo_l, wi_l, mat);
-              const float bp = bsdf_pdf<kOpaque>(wo_l, wi_l, mat);
-              const float cs = wi_l.z;
-              // cpu_tiled.cpp:166-183 divides by a 1e8 "pdf" (the sun then adds ~1e-8 of its
-              // light); XB_FLAG_SUN_NEE weighs the delta light by its pick probability alone,
-              // with MIS weight 1 (no BSDF sample can hit a direction)
-              const float lpdf = sc.sun_nee ? dpick : 1e8f * dpick;
-              const float mis = sc.sun_nee ? 1.f : mis_power2(lpdf, bp);
-              const V3 org = offset_origin(fh.pos, fh.geo_normal, sdir, kShadowEps);
-              const V3 em = v3(sun.emission[0], sun.emission[1], sun.emission[2]);
-              const V3 c = tp * f * cs * (em / lpdf) * mis;
-              s_o = make_float4(org.x, org.y, org.z, kInf);
-              s_d = make_float4(sdir.x, sdir.y, sdir.z, __int_as_float(pid));
-              s_c = make_float4(c.x, c.y, c.z, 0.f);
-              emit_sun = true;
-            }
-          }
-        }
-        if (last) break;   // the reference samples once more, but nothing of it is ever used
-        // ── Russian roulette (cpu_tiled.cpp:190-194) ──
-        if (a.depth >= a.min_bounces) {
-          const float p = smax(0.05f, max_component(tp));
-          if (rng.next_float() > p) break;
-          tp = tp / p;
-        }
-        // ── BSDF sampling and the next ray (cpu_tiled.cpp:197-216) ──
-        const Onb onb(fh.normal);
-        const V3 wo_l = onb.to_local(-ray.d);
+        const bool nee = pass != PASS_NEXT;
+        if (nee ? (mat.flags & kMatDelta) != 0 : last) break;
+        const Onb onb(nee ? fh.geo_normal : fh.normal);
+        const V3 wo_l = onb.to_local(wo);
+        const uint32_t fl = lobe_flags<kOpaque>(mat);
+        float fo = 0.f;
+        if (!kOpaque && (fl & kMatTransmissive))
+          fo = fresnel_dielectric(!nee && (fl & kMatDelta) ? wo_l.z : fabsf(wo_l.z), mat.ior);
+        NeeLight nl;
         BsdfSample s;
-        if (!bsdf_sample<kOpaque>(wo_l, mat, rng, s)) break;
-        if (s.delta) {
-          tp = tp * s.f;
+        int lobe;
+        float scale = 1.f;
+        if (nee) {
+          if (!(pass == PASS_AREA ? area_light(sc, fh.pos, rng, nl) : sun_light(sc, rng, nl))) break;
+          s.wi = onb.to_local(nl.wi);
+          s.delta = false;
+          if (!(s.wi.z > 1e-6f)) break;
+          lobe = nee_lobe<kOpaque>(mat);
         } else {
-          const float ci = fabsf(s.wi.z);
-          if (s.pdf < 1e-8f || ci < 1e-8f) break;
-          tp = tp * (s.f * ci / s.pdf);
+          // Russian roulette (cpu_tiled.cpp:190-194)
+          if (a.depth >= a.min_bounces) {
+            const float p = smax(0.05f, max_component(tp));
+            if (rng.next_float() > p) break;
+            tp = tp / p;
+          }
+          if (!sample_direction<kOpaque>(wo_l, mat, fo, rng, s, lobe, scale)) break;
         }
-        const V3 wiw = onb.to_world(s.wi);
-        const V3 org = offset_origin(fh.pos, fh.geo_normal, wiw, kRayEps);
-        n_o = make_float4(org.x, org.y, org.z, kRayEps);
-        n_d = make_float4(wiw.x, wiw.y, wiw.z, kInf);
-        n_tp = make_float4(tp.x, tp.y, tp.z, s.delta ? -1.f : s.pdf);
-        n_rng = rng.state;
-        emit_next = true;
+        if (lobe == kLobeMfr) mfr_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
+        if (!kOpaque && lobe == kLobeMft) mft_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
+        if (nee) {
+          nee_combine<kOpaque>(s.wi, mat, fo, s.f, s.pdf);
+          // cpu_tiled.cpp:166-183 divides a sun by a 1e8 "pdf" (it then adds ~1e-8 of its light);
+          // XB_FLAG_SUN_NEE weighs the delta light by its pick probability alone, with MIS
+          // weight 1 (no BSDF sample can hit a direction)
+          const float mis = pass == PASS_SUN && sc.sun_nee ? 1.f : mis_power2(nl.pdf, s.pdf);
+          if (pass == PASS_AREA && !(mis > 0.0f && nl.pdf > 1e-12f)) break;
+          const V3 org = offset_origin(fh.pos, fh.geo_normal, nl.wi, kShadowEps);
+          const V3 c = tp * s.f * s.wi.z * (nl.emission / nl.pdf) * mis;
+          q_o = make_float4(org.x, org.y, org.z, nl.tmax);
+          q_d = make_float4(nl.wi.x, nl.wi.y, nl.wi.z, __int_as_float(pid));
+          q_c = make_float4(c.x, c.y, c.z, 0.f);
+        } else {
+          if (lobe != kLobeNone && s.pdf < 1e-8f) break;
+          if (s.delta) {
+            tp = tp * s.f;
+          } else {
+            s.pdf *= scale;
+            const float ci = fabsf(s.wi.z);
+            if (s.pdf < 1e-8f || ci < 1e-8f) break;
+            tp = tp * (s.f * ci / s.pdf);
+          }
+          const V3 wiw = onb.to_world(s.wi);
+          const V3 org = offset_origin(fh.pos, fh.geo_normal, wiw, kRayEps);
+          q_o = make_float4(org.x, org.y, org.z, kRayEps);
+          q_d = make_float4(wiw.x, wiw.y, wiw.z, kInf);
+          q_c = make_float4(tp.x, tp.y, tp.z, s.delta ? -1.f : s.pdf);
+        }
+        emit = true;
       } while (false);
+      int32_t* const counter = pass == PASS_NEXT ? a.cnt_next + CNT_RAYS : a.cnt + (pass == PASS_AREA ? CNT_SH_AREA : CNT_SH_SUN);
+      const int idx = warp_append(counter, emit, a.capacity, a.stats + STAT_OVERFLOW);
+      if (idx >= 0) {
+        if (pass == PASS_NEXT) {
+          a.nray_o[idx] = q_o; a.nray_d[idx] = q_d; a.ntp[idx] = q_c;
+          a.nrng[idx] = rng.state;
+          a.npath[idx] = pid;
+        } else {
+          const int k = pass == PASS_AREA ? 0 : 1;
+          a.sh_o[k][idx] = q_o; a.sh_d[k][idx] = q_d; a.sh_c[k][idx] = q_c;
+        }
+      }
     }
-    int idx = warp_append(a.cnt_next + CNT_RAYS, emit_next, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) {
-      a.nray_o[idx] = n_o; a.nray_d[idx] = n_d; a.ntp[idx] = n_tp; a.nrng[idx] = n_rng;
-      a.npath[idx] = pid;
-    }
-    idx = warp_append(a.cnt + CNT_SH_AREA, emit_area, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) { a.sh_o[0][idx] = a_o; a.sh_d[0][idx] = a_d; a.sh_c[0][idx] = a_c; }
-    idx = warp_append(a.cnt + CNT_SH_SUN, emit_sun, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) { a.sh_o[1][idx] = s_o; a.sh_d[1][idx] = s_d; a.sh_c[1][idx] = s_c; }
   }
 }
 
