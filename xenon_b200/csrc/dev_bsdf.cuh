@@ -168,25 +168,34 @@ __device__ __forceinline__ float mfr_pdf(V3 wo, V3 wi, const DevMaterial& m) {
   float jac = 1.f / (4.f * fabsf(dot(wo, wh)));
   return dv * jac;
 }
-// mfr_eval and mfr_pdf of one pair of directions: the same operations, the half vector, the
-// distribution and Lambda(wo) computed once.
-__device__ __forceinline__ void mfr_eval_pdf(V3 wo, V3 wi, const DevMaterial& m, V3& f, float& pdf) {
-  f = v3s(0.f);
-  pdf = 0.f;
-  if (wo.z <= 0.f || wi.z <= 0.f) return;
+// mfr_pdf of one pair of directions, and mfr_eval from what the two share (the half vector, the
+// distribution, Lambda(wo)): the same operations, each once. pdf, whz and d are 0 where mfr_pdf
+// returns early.
+struct MfrHalf {
+  float pdf, whz, d, lo, dwo;
+};
+__device__ __forceinline__ MfrHalf mfr_half(V3 wo, V3 wi, const DevMaterial& m) {
+  MfrHalf h{0.f, 0.f, 0.f, 0.f, 0.f};
+  if (wo.z <= 0.f || wi.z <= 0.f) return h;
   const V3 wh = normalize(wo + wi);
-  if (wh.z <= 0.f) return;
-  const float d = ggx_d_aniso(wh, m.alpha_x, m.alpha_y);
-  const float lo = ggx_lambda_aniso(wo, m.alpha_x, m.alpha_y), li = ggx_lambda_aniso(wi, m.alpha_x, m.alpha_y);
-  const float dwo = dot(wo, wh);
-  const float denom = 4.f * wo.z * wi.z;
-  if (!(denom < 1e-8f)) {
-    f = mf_fresnel(dwo, m) * d * (1.f / (1.f + lo + li)) / denom;
-    if (!(m.flags & kMatTransmissive)) f = f * multiscatter(m, wo.z, wi.z);
-  }
+  if (wh.z <= 0.f) return h;
+  h.whz = wh.z;
+  h.d = ggx_d_aniso(wh, m.alpha_x, m.alpha_y);
+  h.lo = ggx_lambda_aniso(wo, m.alpha_x, m.alpha_y);
+  h.dwo = dot(wo, wh);
   const float co = fabsf(wo.z);
-  const float dv = co < 1e-8f ? 0.f : d * (1.f / (1.f + lo)) * smax(0.f, dwo) / co;
-  pdf = dv * (1.f / (4.f * fabsf(dwo)));
+  const float dv = co < 1e-8f ? 0.f : h.d * (1.f / (1.f + h.lo)) * smax(0.f, h.dwo) / co;
+  h.pdf = dv * (1.f / (4.f * fabsf(h.dwo)));
+  return h;
+}
+__device__ __forceinline__ V3 mfr_eval(V3 wo, V3 wi, const DevMaterial& m, const MfrHalf& h) {
+  const float denom = 4.f * wo.z * wi.z;
+  // a half vector of NaN components passes mfr_half's test, as it does mfr_eval's
+  if (wo.z <= 0.f || wi.z <= 0.f || h.whz == 0.f || denom < 1e-8f) return v3s(0.f);
+  const float li = ggx_lambda_aniso(wi, m.alpha_x, m.alpha_y);
+  V3 f = mf_fresnel(h.dwo, m) * h.d * (1.f / (1.f + h.lo + li)) / denom;
+  if (!(m.flags & kMatTransmissive)) f = f * multiscatter(m, wo.z, wi.z);
+  return f;
 }
 __device__ __forceinline__ bool mfr_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample& s) {
   if (wo.z <= 0.f) return false;
@@ -239,7 +248,7 @@ __device__ __forceinline__ float mft_pdf(V3 wo, V3 wi, const DevMaterial& m) {
   float dwh = fabsf((eta * eta * dwi) / (denom * denom));
   return pwh * dwh;
 }
-// mft_eval and mft_pdf of one pair of directions, as mfr_eval_pdf.
+// mft_eval and mft_pdf of one pair of directions, as mfr_half and mfr_eval.
 __device__ __forceinline__ void mft_eval_pdf(V3 wo, V3 wi, const DevMaterial& m, V3& fv, float& pdf) {
   fv = v3s(0.f);
   pdf = 0.f;
@@ -348,26 +357,8 @@ __device__ __forceinline__ bool cosine_sample(V3 wo, V3 color, const DevMaterial
 }
 
 // ── combined eval / pdf for NEE (bsdf.h:601-657) ───────────────────────────────
-// The three entry points the bounce kernels call: inlined (the default build) or, built with
-// XB_BSDF_CALLS, kept as calls so that a bounce kernel holds one copy of each body (its two NEE
-// sites evaluate the BSDF) — less code for the instruction cache, more register traffic at the calls.
-#ifdef XB_BSDF_CALLS
-#define XB_BSDF_ENTRY __device__ __noinline__
-#else
-#define XB_BSDF_ENTRY __device__ __forceinline__
-#endif
-
-// kOpaque: the scene has no delta, transmissive or subsurface material (the renderer checks at
-// upload), so those branches are left out of the bounce kernel's code; the same arithmetic runs
-// for every material it does have.
-template <bool kOpaque>
-__device__ __forceinline__ uint32_t lobe_flags(const DevMaterial& m) {
-  return kOpaque ? (m.flags & kMatConductor) : m.flags;
-}
-
-template <bool kOpaque = false>
-XB_BSDF_ENTRY V3 bsdf_eval(V3 wo, V3 wi, const DevMaterial& m) {
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+__device__ __forceinline__ V3 bsdf_eval(V3 wo, V3 wi, const DevMaterial& m) {
+  const uint32_t fl = m.flags;
   if (fl & kMatDelta) return v3s(0.f);
   if (fl & kMatConductor) return mfr_eval(wo, wi, m);
   if (fl & kMatTransmissive) return (wi.z > 0.f) ? mfr_eval(wo, wi, m) : mft_eval(wo, wi, m);
@@ -381,9 +372,8 @@ XB_BSDF_ENTRY V3 bsdf_eval(V3 wo, V3 wi, const DevMaterial& m) {
   return v3s(0.f);
 }
 
-template <bool kOpaque = false>
-XB_BSDF_ENTRY float bsdf_pdf(V3 wo, V3 wi, const DevMaterial& m) {
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+__device__ __forceinline__ float bsdf_pdf(V3 wo, V3 wi, const DevMaterial& m) {
+  const uint32_t fl = m.flags;
   if (fl & kMatDelta) return 0.f;
   if (fl & kMatConductor) return mfr_pdf(wo, wi, m);
   if (fl & kMatTransmissive) {
@@ -399,13 +389,12 @@ XB_BSDF_ENTRY float bsdf_pdf(V3 wo, V3 wi, const DevMaterial& m) {
 }
 
 // ── lobe selection and sampling (bsdf.h:666-708) ───────────────────────────────
-template <bool kOpaque = false>
-XB_BSDF_ENTRY bool bsdf_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample& s) {
+__device__ __forceinline__ bool bsdf_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample& s) {
   s.delta = false;
   s.pdf = 0.f;
   s.f = v3s(0.f);
   s.wi = v3s(0.f);
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+  const uint32_t fl = m.flags;
   if (fl & kMatDelta) {
     if (fl & kMatTransmissive) {
       float f = fresnel_dielectric(wo.z, m.ior);
@@ -445,19 +434,24 @@ XB_BSDF_ENTRY bool bsdf_sample(V3 wo, const DevMaterial& m, Pcg& rng, BsdfSample
 // kernel of 287 KB of code whose warps waited 43 to 79 cycles per instruction for the instruction
 // cache; the kernels therefore loop over the three with one copy of the evaluation between the
 // lobe choice (before) and the combination (after).
+// kKinds: the material flags that can occur (the renderer checks a scene's at upload); the code of
+// the others is left out, and the same arithmetic runs for every material there is.
 enum { kLobeNone = 0, kLobeMfr = 1, kLobeMft = 2 };
+constexpr uint32_t kAllKinds = kMatConductor | kMatTransmissive | kMatSubsurface | kMatDelta;
+constexpr uint32_t kOpaqueKinds = kMatConductor;
+constexpr uint32_t kGuidedKinds = kMatConductor | kMatSubsurface;
 
 // The lobe that next-event estimation evaluates (wi.z > 0, not a delta material).
-template <bool kOpaque>
+template <uint32_t kKinds>
 __device__ __forceinline__ int nee_lobe(const DevMaterial& m) {
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+  const uint32_t fl = m.flags & kKinds;
   return (fl & kMatSubsurface) && !(fl & (kMatConductor | kMatTransmissive)) ? kLobeNone : kLobeMfr;
 }
 // bsdf_eval and bsdf_pdf for wi.z > 0 from the lobe's f and pdf; fo: fresnel_dielectric(|wo.z|) of a
 // transmissive material.
-template <bool kOpaque>
+template <uint32_t kKinds>
 __device__ __forceinline__ void nee_combine(V3 wi, const DevMaterial& m, float fo, V3& f, float& pdf) {
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+  const uint32_t fl = m.flags & kKinds;
   if (fl & kMatConductor) return;
   if (fl & kMatTransmissive) {
     pdf = fo * pdf;
@@ -476,7 +470,7 @@ __device__ __forceinline__ void nee_combine(V3 wi, const DevMaterial& m, float f
 
 // bsdf_sample up to the evaluation: the lobe, its direction and the factor of its pdf. With lobe
 // kLobeNone s is complete but for that factor. False where bsdf_sample fails before it evaluates.
-template <bool kOpaque>
+template <uint32_t kKinds>
 __device__ __forceinline__ bool sample_direction(V3 wo, const DevMaterial& m, float fo, Pcg& rng, BsdfSample& s,
                                                  int& lobe, float& scale) {
   s.delta = false;
@@ -485,7 +479,7 @@ __device__ __forceinline__ bool sample_direction(V3 wo, const DevMaterial& m, fl
   s.wi = v3s(0.f);
   lobe = kLobeMfr;
   scale = 1.f;
-  const uint32_t fl = lobe_flags<kOpaque>(m);
+  const uint32_t fl = m.flags & kKinds;
   if (fl & kMatDelta) {
     lobe = kLobeNone;
     if ((fl & kMatTransmissive) && !(rng.next_float() < fo)) return delta_trans_sample(wo, m, s);
@@ -549,6 +543,9 @@ __device__ __forceinline__ bool sample_direction(V3 wo, const DevMaterial& m, fl
 // elsewhere by the sampler's density, which must be the true one.
 __device__ __forceinline__ float cos4(float c) { const float c2 = c * c; return c2 * c2; }
 
+// From mfr_half's pdf and half vector.
+__device__ __forceinline__ float mfr_density(float pdf, float whz) { return pdf > 0.f ? pdf * cos4(whz) : 0.f; }
+
 __device__ __forceinline__ float mfr_density(V3 wo, V3 wi, const DevMaterial& m) {
   const float p = mfr_pdf(wo, wi, m);
   if (!(p > 0.f)) return 0.f;
@@ -557,34 +554,42 @@ __device__ __forceinline__ float mfr_density(V3 wo, V3 wi, const DevMaterial& m)
 
 // For a non-delta, non-transmissive material seen from its front side (wo.z > 0), bsdf_sample
 // draws a lobe l with probability P_l and a direction from that lobe, returning f_l and its
-// stated P_l pdf_l. Given a direction wi drawn by another proposal, this returns what the sampler
-// would have returned had it produced wi — a lobe chosen with its posterior P_l d_l(wi) /
-// sum_k P_k d_k(wi) (d: true densities; u selects it), that lobe's f and stated P_l pdf_l — and
-// the sampler's true marginal density sum_k P_k d_k(wi). Returns false where the sampler cannot
-// produce wi.
-__device__ __forceinline__ bool bsdf_lobe_for_direction(V3 wo, V3 wi, const DevMaterial& m, float u, V3& f,
-                                                        float& pdf_sel, float& density) {
+// stated P_l pdf_l. guided_density returns the sampler's true marginal density sum_k P_k d_k(wi) of
+// a direction wi (d: true densities), given mfr_half's values for it (not read for a subsurface
+// material). guided_lobe does what the sampler would have returned had it produced a direction wi
+// that another proposal drew: a lobe chosen with its posterior P_l d_l(wi) / sum_k P_k d_k(wi) (u
+// selects it), that lobe's f (of a microfacet lobe: left to mfr_eval) and stated P_l pdf_l. False
+// where the sampler cannot produce wi.
+__device__ __forceinline__ bool guided_needs_mfr(const DevMaterial& m) {
+  return (m.flags & kMatConductor) || !(m.flags & kMatSubsurface);
+}
+__device__ __forceinline__ float guided_density(V3 wi, const DevMaterial& m, const MfrHalf& h) {
+  if (m.flags & kMatConductor) return mfr_density(h.pdf, h.whz);
+  if (m.flags & kMatSubsurface) return diffuse_pdf(wi);
+  const float spec = sclamp(m.f0[0], 0.f, 1.f);
+  return spec * mfr_density(h.pdf, h.whz) + (1.f - spec) * diffuse_pdf(wi);
+}
+__device__ __forceinline__ bool guided_lobe(V3 wi, const DevMaterial& m, float u, const MfrHalf& h, float density,
+                                            int& lobe, BsdfSample& s) {
+  lobe = kLobeNone;
   if (m.flags & kMatConductor) {
-    pdf_sel = mfr_pdf(wo, wi, m);
-    density = mfr_density(wo, wi, m);
-    f = mfr_eval(wo, wi, m);
+    s.pdf = h.pdf;
+    lobe = kLobeMfr;
   } else if (m.flags & kMatSubsurface) {
-    pdf_sel = density = diffuse_pdf(wi);
-    f = (wi.z > 0.f) ? ss_color(m) * (1.f - m.metallic) * kInvPi : v3s(0.f);
+    s.pdf = density;
+    s.f = (wi.z > 0.f) ? ss_color(m) * (1.f - m.metallic) * kInvPi : v3s(0.f);
   } else {
-    const float spec = sclamp(m.f0[0], 0.f, 1.f), diff = 1.f - spec;
-    const float ds = spec * mfr_density(wo, wi, m), dd = diff * diffuse_pdf(wi);
-    density = ds + dd;
     if (!(density > 0.f)) return false;
-    if (u * density < ds) {
-      pdf_sel = spec * mfr_pdf(wo, wi, m);
-      f = mfr_eval(wo, wi, m);
+    const float spec = sclamp(m.f0[0], 0.f, 1.f), diff = 1.f - spec;
+    if (u * density < spec * mfr_density(h.pdf, h.whz)) {
+      s.pdf = spec * h.pdf;
+      lobe = kLobeMfr;
     } else {
-      pdf_sel = dd;
-      f = diffuse_eval(wi, m);
+      s.pdf = diff * diffuse_pdf(wi);
+      s.f = diffuse_eval(wi, m);
     }
   }
-  return pdf_sel >= 1e-8f && density > 0.f;
+  return s.pdf >= 1e-8f && density > 0.f;
 }
 
 // The true density with which bsdf_sample (front side; non-delta, non-transmissive material)

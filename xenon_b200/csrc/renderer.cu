@@ -428,6 +428,7 @@ enum { PASS_AREA = 0, PASS_SUN = 1, PASS_NEXT = 2 };
 // 0.47 / 0.51 / 0.62.
 template <int kOcc, bool kOpaque>
 __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
+  constexpr uint32_t kKinds = kOpaque ? kOpaqueKinds : kAllKinds;
   const int n = a.cnt[CNT_RAYS];
   const DevScene& sc = a.sc;
   const bool last_all = (a.depth + 1 >= a.max_bounces);
@@ -473,9 +474,9 @@ __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
         if (nee ? (mat.flags & kMatDelta) != 0 : last) break;
         const Onb onb(nee ? fh.geo_normal : fh.normal);
         const V3 wo_l = onb.to_local(wo);
-        const uint32_t fl = lobe_flags<kOpaque>(mat);
+        const uint32_t fl = mat.flags & kKinds;
         float fo = 0.f;
-        if (!kOpaque && (fl & kMatTransmissive))
+        if (fl & kMatTransmissive)
           fo = fresnel_dielectric(!nee && (fl & kMatDelta) ? wo_l.z : fabsf(wo_l.z), mat.ior);
         NeeLight nl;
         BsdfSample s;
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
           s.wi = onb.to_local(nl.wi);
           s.delta = false;
           if (!(s.wi.z > 1e-6f)) break;
-          lobe = nee_lobe<kOpaque>(mat);
+          lobe = nee_lobe<kKinds>(mat);
         } else {
           // Russian roulette (cpu_tiled.cpp:190-194)
           if (a.depth >= a.min_bounces) {
@@ -494,12 +495,16 @@ __global__ void __launch_bounds__(128, kOcc) shade_kernel(ShadeArgs a) {
             if (rng.next_float() > p) break;
             tp = tp / p;
           }
-          if (!sample_direction<kOpaque>(wo_l, mat, fo, rng, s, lobe, scale)) break;
+          if (!sample_direction<kKinds>(wo_l, mat, fo, rng, s, lobe, scale)) break;
         }
-        if (lobe == kLobeMfr) mfr_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
-        if (!kOpaque && lobe == kLobeMft) mft_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
+        if (lobe == kLobeMfr) {
+          const MfrHalf h = mfr_half(wo_l, s.wi, mat);
+          s.pdf = h.pdf;
+          s.f = mfr_eval(wo_l, s.wi, mat, h);
+        }
+        if ((kKinds & kMatTransmissive) && lobe == kLobeMft) mft_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
         if (nee) {
-          nee_combine<kOpaque>(s.wi, mat, fo, s.f, s.pdf);
+          nee_combine<kKinds>(s.wi, mat, fo, s.f, s.pdf);
           // cpu_tiled.cpp:166-183 divides a sun by a 1e8 "pdf" (it then adds ~1e-8 of its light);
           // XB_FLAG_SUN_NEE weighs the delta light by its pick probability alone, with MIS
           // weight 1 (no BSDF sample can hit a direction)
@@ -583,6 +588,19 @@ __device__ __forceinline__ float capped_selection(float a, float ratio, float ca
 }
 
 constexpr float kNaN = __builtin_nanf("");
+
+// One training record: the vertex's features, the direction, the actual throughput before it and
+// the BSDF sampler's density; the path radiance before its continuation is set by the next bounce.
+__device__ __forceinline__ void write_record(float* recs, int i, const float* feat, V3 wi, int32_t pid, V3 tb,
+                                             float pb) {
+  float4* R = reinterpret_cast<float4*>(recs + (size_t)i * xbg::kRecFloats);
+  R[0] = make_float4(feat[0], feat[1], feat[2], feat[3]);
+  R[1] = make_float4(feat[4], feat[5], feat[6], feat[7]);
+  R[2] = make_float4(feat[8], wi.x, wi.y, wi.z);
+  R[3] = make_float4(0.f, __int_as_float(pid), tb.x, tb.y);
+  R[4] = make_float4(tb.z, kNaN, kNaN, kNaN);
+  R[5] = make_float4(pb, 0.f, 0.f, 0.f);
+}
 constexpr int kLobStride = xbg::kLobeFloats + 1;   // conflict-free per-thread rows
 // The lobes of a tile's rows take the activation tile's place once its last layer has run.
 constexpr size_t kLobBytes = (size_t)xbg::kTile * kLobStride * 4;
@@ -594,6 +612,11 @@ constexpr size_t kGuidedShadeSmem =
 // same bounce past the bounces the network serves (xb_guiding.guided_bounces): every vertex
 // samples its BSDF, the importance ratio of the path's earlier guided vertices is carried on, and
 // there is no network, shared memory or barrier, so it launches like the plain bounce.
+// Its code and the network pass's were 455 and 210 KB before the passes around one evaluation (see
+// dev_bsdf.cuh). B200, both kernels, ms per sample at 1080p / 720p: 261 instances of every material
+// kind 4.05 -> 1.61, the room of one diffuse material 1.28 -> 1.23; the fused form, whose atomics
+// now lie on a tile's serial chain, 1.48 -> 1.82 in the room and 6.4 -> 3.4 (whole render) with the
+// instances.
 template <bool kNet, int kOcc>
 __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(ShadeArgs a, GuideShadeArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -616,25 +639,19 @@ __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(Shad
   float* lob = sLob + threadIdx.x * kLobStride;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int slot = base + threadIdx.x;
-    bool emit_next = false, emit_area = false, emit_sun = false, emit_rec = false, emit_defer = false;
-    float4 n_o, n_d, n_tp;
-    uint64_t n_rng = 0;
-    int32_t pid = 0;
-    float n_ratio = 1.f;
-    float4 a_o, a_d, a_c, s_o, s_d, s_c;
-    float4 rec[6];
-    float4 dq[5];
     // ── phase 1: emitter test and the network's input ──
-    bool alive = false, guided = false;
+    bool alive = false, guided = false, last = last_all;
+    int32_t pid = 0;
     float feat[9] = {0.5f, 0.5f, 0.5f, 0.f, 0.f, 1.f, 0.f, 0.f, 1.f};
-    float4 ro = make_float4(0, 0, 0, 0), rd = ro, tpv = ro;
+    V3 tp = v3s(0.f), wo = v3s(0.f);   // tp: the plain estimator's throughput
     float ratio = 1.f;
     Pcg rng{0};
     FullHit fh;
     fh.mat_id = 0;
     if (slot < n) {
-      ro = a.ray_o[slot]; rd = a.ray_d[slot]; tpv = a.tp[slot];
+      const float4 ro = a.ray_o[slot], rd = a.ray_d[slot], tpv = a.tp[slot];
       pid = a.path[slot];
+      if (a.path_maxd) last = a.depth + 1 >= (int)a.path_maxd[pid];
       rng.state = a.rng[slot];
       if (g.ratio_in) ratio = g.ratio_in[slot];
       if (g.rec_in) {
@@ -646,36 +663,20 @@ __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(Shad
         }
       }
       const Ray ray{v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z), ro.w, rd.w};
-      const V3 tpr = v3(tpv.x, tpv.y, tpv.z) * ratio;   // the path's actual throughput
+      tp = v3(tpv.x, tpv.y, tpv.z);
+      wo = -ray.d;
+      const V3 tpr = tp * ratio;   // the path's actual throughput
       const float4 hv = a.hit[slot];
       const int hinst = a.hit_inst[slot];
       if (hinst < 0) {
         if (sc.sky_intensity > 0.f) add_L(a.L, pid, tpr * sky_eval(sc, ray.d));
       } else {
-        HitState h{hv.x, hv.y, hv.z, __float_as_int(hv.w), hinst};
+        const HitState h{hv.x, hv.y, hv.z, __float_as_int(hv.w), hinst};
         complete_hit(sc, ray, h, fh);
-        bool hit_light = false;
-        for (int li = 0; li < sc.num_lights; ++li) {
-          const DevLight& lt = sc.lights[li];
-          if (__float_as_int(lt.p2.w) == fh.prim_id && __float_as_int(lt.p1.w) == fh.instance_id) {
-            float mis = 1.0f;
-            const float cos_l = smax(0.0f, dot(fh.geo_normal, -ray.d));
-            if (cos_l > 1e-6f) {
-              if (a.depth > 0 && !(tpv.w < 0.f)) {
-                const float pdf_area = (1.0f / lt.p0.w) * (1.0f / (float)sc.num_lights);
-                const float pdf_sa = (pdf_area * (h.t * h.t)) / cos_l;
-                mis = mis_power2(tpv.w, pdf_sa);
-              }
-              add_L(a.L, pid, tpr * v3(lt.emission.x, lt.emission.y, lt.emission.z) * mis);
-            }
-            hit_light = true;
-            break;
-          }
-        }
-        if (!hit_light) {
-          alive = true;
+        alive = !emitter_hit(a, fh, wo, h.t, tpr, tpv.w, pid);
+        if (alive) {
           // The network proposes at non-delta, non-transmissive vertices seen from the front of
-          // the shading normal, where the density of bsdf_sample is known (bsdf_density);
+          // the shading normal, where the density of bsdf_sample is known (guided_density);
           // elsewhere the plain sampler runs. Rough dielectrics stay plain: the reference
           // evaluates their transmission with a half vector (wo + wi / ior) other than the one
           // its sampler refracts about (and its pdf can be NaN there), so neither its pdf nor a
@@ -687,13 +688,13 @@ __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(Shad
           const uint32_t mf = gm.flags;
           const bool proposal = kNet || g.gq[0] != nullptr ||
                                 (g.sky_alpha > 0.f && (!(mf & kMatConductor) || gm.alpha >= 0.25f));
-          guided = proposal && (mf & (kMatDelta | kMatTransmissive)) == 0 && dot(fh.normal, -ray.d) > 0.f;
+          guided = proposal && (mf & (kMatDelta | kMatTransmissive)) == 0 && dot(fh.normal, wo) > 0.f;
           for (int k = 0; k < 3; ++k) {
             const float pk = (k == 0 ? fh.pos.x : k == 1 ? fh.pos.y : fh.pos.z);
             feat[k] = fminf(fmaxf((pk - g.bmin[k]) * g.binv[k], 0.f), 1.f);
           }
           feat[3] = fh.normal.x; feat[4] = fh.normal.y; feat[5] = fh.normal.z;
-          feat[6] = -ray.d.x; feat[7] = -ray.d.y; feat[8] = -ray.d.z;
+          feat[6] = wo.x; feat[7] = wo.y; feat[8] = wo.z;
         }
       }
     }
@@ -709,185 +710,155 @@ __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(Shad
       xbg::raw_to_lobes<true>(raw, lob);
       alpha = g.alpha >= 0.f ? g.alpha : xbg::selection<true>(raw);
     }
-    // ── phase 2: NEE, roulette, the next direction (cpu_tiled.cpp:89-216) ──
-    if (alive) do {
-      const Ray ray{v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z), ro.w, rd.w};
-      V3 tp = v3(tpv.x, tpv.y, tpv.z);   // the plain estimator's throughput
-      const DevMaterial& mat = sc.mats[fh.mat_id];
-      const bool is_delta = (mat.flags & kMatDelta) != 0;
-      if (sc.num_lights > 0 && !is_delta) {
-        const float upick = rng.next_float();
-        int li = (int)(upick * (float)sc.num_lights);
-        li = li < 0 ? 0 : (li > sc.num_lights - 1 ? sc.num_lights - 1 : li);
-        const float pick_pdf = 1.f / (float)sc.num_lights;
-        const DevLight& lt = sc.lights[li];
-        const float u1 = rng.next_float();
-        const float u2 = rng.next_float();
-        const float su1 = sqrtf(u1);
-        const float b0 = 1.0f - su1;
-        const float b1 = u2 * su1;
-        const float b2 = 1.0f - b0 - b1;
-        const V3 lp = ld3(lt.p0) * b0 + ld3(lt.p1) * b1 + ld3(lt.p2) * b2;
-        const V3 sdir = lp - fh.pos;
-        const float dsq = length_sq(sdir);
-        const float dist = sqrtf(dsq);
-        if (dist > 1e-6f) {
-          const V3 wi = sdir / dist;
-          const float cos_l = smax(0.0f, dot(ld3(lt.n), -wi));
-          const Onb onb(fh.geo_normal);
-          const V3 wo_l = onb.to_local(-ray.d);
-          const V3 wi_l = onb.to_local(wi);
-          if (cos_l > 1e-6f && wi_l.z > 1e-6f) {
-            const V3 f = bsdf_eval(wo_l, wi_l, mat);
-            const float bp = bsdf_pdf(wo_l, wi_l, mat);
-            const float lpdf = ((1.0f / lt.p0.w) * pick_pdf) * (dsq / cos_l);
-            const float mis = mis_power2(lpdf, bp);
-            if (mis > 0.0f && lpdf > 1e-12f) {
-              const V3 org = offset_origin(fh.pos, fh.geo_normal, wi, kShadowEps);
-              const V3 c = (tp * ratio) * f * wi_l.z * (v3(lt.emission.x, lt.emission.y, lt.emission.z) / lpdf) * mis;
-              a_o = make_float4(org.x, org.y, org.z, dist - kShadowEps);
-              a_d = make_float4(wi.x, wi.y, wi.z, __int_as_float(pid));
-              a_c = make_float4(c.x, c.y, c.z, 0.f);
-              emit_area = true;
+    // ── phase 2: NEE, roulette, the next direction (cpu_tiled.cpp:89-216), in passes around one
+    // evaluation as shade_kernel's ──
+#pragma unroll 1
+    for (int pass = PASS_AREA; pass <= PASS_NEXT; ++pass) {
+      if (pass == PASS_AREA && sc.num_lights == 0) continue;
+      if (pass == PASS_SUN && sc.num_suns == 0) continue;
+      if (pass == PASS_NEXT && last_all) break;
+      bool emit = false, emit_rec = false, emit_defer = false;
+      float4 q_o, q_d, q_c;
+      float n_ratio = 1.f, pb = 0.f;
+      V3 tb = v3s(0.f);   // actual throughput before the vertex's scattering
+      if (alive) do {
+        const DevMaterial& mat = sc.mats[fh.mat_id];
+        const bool nee = pass != PASS_NEXT;
+        if (nee ? (mat.flags & kMatDelta) != 0 : last) break;
+        const Onb onb(nee ? fh.geo_normal : fh.normal);
+        const V3 wo_l = onb.to_local(wo);
+        float fo = 0.f;
+        if (mat.flags & kMatTransmissive)
+          fo = fresnel_dielectric(!nee && (mat.flags & kMatDelta) ? wo_l.z : fabsf(wo_l.z), mat.ior);
+        NeeLight nl;
+        BsdfSample s;
+        V3 wiw;
+        int lobe = kLobeNone;
+        float scale = 1.f, ap = 0.f, u_lobe = 0.f;
+        bool proposed = false;
+        if (nee) {
+          if (!(pass == PASS_AREA ? area_light(sc, fh.pos, rng, nl) : sun_light(sc, rng, nl))) break;
+          s.wi = onb.to_local(nl.wi);
+          s.delta = false;
+          if (!(s.wi.z > 1e-6f)) break;
+          lobe = nee_lobe<kAllKinds>(mat);
+        } else {
+          if (a.depth >= a.min_bounces) {
+            // cpu_tiled.cpp:190-194 on the plain throughput: p = max(0.05, max(tp)), survive with
+            // min(1, p), divide by p. Its part above 1 is a deterministic rescale and stays as is;
+            // the survival draw is made with the probability the actual throughput (tp * ratio)
+            // asks for, and the ratio of the two survival probabilities joins the importance ratio.
+            const float p = smax(0.05f, max_component(tp));
+            const float surv = smin(1.f, p);
+            const float surv_g = sclamp(max_component(tp * ratio) / smax(1.f, p), 0.05f, 1.f);
+            if (rng.next_float() > surv_g) break;
+            tp = tp / p;
+            ratio = ratio * (surv / surv_g);
+          }
+          if (!kNet && guided && g.gq[0] != nullptr) {
+            emit_defer = true;   // two-kernel form: the network pass samples this vertex's direction
+            break;
+          }
+          if (guided) {
+            // the proposal: the network's mixture (kNet) or the sky's luminance distribution
+            ap = capped_selection(kNet ? alpha : g.sky_alpha, ratio, g.ratio_cap);
+            if (rng.next_float() < ap) {
+              if constexpr (kNet) {
+                const float u0 = rng.next_float(), u1 = rng.next_float(), u2 = rng.next_float();
+                float d[3];
+                xbg::mix_sample(lob, u0, u1, u2, d);
+                wiw = v3(d[0], d[1], d[2]);
+              } else {
+                const float u0 = rng.next_float(), u1 = rng.next_float();
+                wiw = sky_sample(sc.sky_cdf, u0, u1);
+              }
+              s.wi = onb.to_local(wiw);
+              s.delta = false;
+              u_lobe = rng.next_float();
+              proposed = true;
             }
           }
-        }
-      }
-      if (sc.num_suns > 0 && !is_delta) {
-        const float upick = rng.next_float();
-        int di = (int)(upick * (float)sc.num_suns);
-        di = di < 0 ? 0 : (di > sc.num_suns - 1 ? sc.num_suns - 1 : di);
-        const float dpick = 1.f / (float)sc.num_suns;
-        const DevSun& sun = sc.suns[di];
-        const V3 sdir = v3(sun.dir[0], sun.dir[1], sun.dir[2]);
-        const Onb onb(fh.geo_normal);
-        const V3 wo_l = onb.to_local(-ray.d);
-        const V3 wi_l = onb.to_local(sdir);
-        if (wi_l.z > 1e-6f) {
-          const V3 f = bsdf_eval(wo_l, wi_l, mat);
-          const float bp = bsdf_pdf(wo_l, wi_l, mat);
-          const float lpdf = sc.sun_nee ? dpick : 1e8f * dpick;   // as in shade_kernel
-          const float mis = sc.sun_nee ? 1.f : mis_power2(lpdf, bp);
-          const V3 org = offset_origin(fh.pos, fh.geo_normal, sdir, kShadowEps);
-          const V3 em = v3(sun.emission[0], sun.emission[1], sun.emission[2]);
-          const V3 c = (tp * ratio) * f * wi_l.z * (em / lpdf) * mis;
-          s_o = make_float4(org.x, org.y, org.z, kInf);
-          s_d = make_float4(sdir.x, sdir.y, sdir.z, __int_as_float(pid));
-          s_c = make_float4(c.x, c.y, c.z, 0.f);
-          emit_sun = true;
-        }
-      }
-      if (a.path_maxd ? (a.depth + 1 >= (int)a.path_maxd[pid]) : last_all) break;
-      if (a.depth >= a.min_bounces) {
-        // cpu_tiled.cpp:190-194 on the plain throughput: p = max(0.05, max(tp)), survive with
-        // min(1, p), divide by p. Its part above 1 is a deterministic rescale and stays as is;
-        // the survival draw is made with the probability the actual throughput (tp * ratio)
-        // asks for, and the ratio of the two survival probabilities joins the importance ratio.
-        const float p = smax(0.05f, max_component(tp));
-        const float surv = smin(1.f, p);
-        const float surv_g = sclamp(max_component(tp * ratio) / smax(1.f, p), 0.05f, 1.f);
-        if (rng.next_float() > surv_g) break;
-        tp = tp / p;
-        ratio = ratio * (surv / surv_g);
-      }
-      if (!kNet && guided && g.gq[0] != nullptr) {
-        // two-kernel form: the network pass samples this vertex's direction
-        dq[0] = make_float4(fh.pos.x, fh.pos.y, fh.pos.z, __int_as_float(fh.mat_id));
-        dq[1] = make_float4(fh.normal.x, fh.normal.y, fh.normal.z, __int_as_float(pid));
-        dq[2] = make_float4(fh.geo_normal.x, fh.geo_normal.y, fh.geo_normal.z, ratio);
-        dq[3] = make_float4(-ray.d.x, -ray.d.y, -ray.d.z, 0.f);
-        dq[4] = make_float4(tp.x, tp.y, tp.z, 0.f);
-        n_rng = rng.state;
-        emit_defer = true;
-        break;
-      }
-      const Onb onb(fh.normal);
-      const V3 wo_l = onb.to_local(-ray.d);
-      BsdfSample s;
-      V3 wiw;
-      n_ratio = ratio;
-      if (!guided) {
-        if (!bsdf_sample(wo_l, mat, rng, s)) break;
-        wiw = onb.to_world(s.wi);
-      } else {
-        // the proposal: the network's mixture (kNet) or the sky's luminance distribution
-        float pb;
-        const float ap = capped_selection(kNet ? alpha : g.sky_alpha, ratio, g.ratio_cap);
-        if (rng.next_float() < ap) {
-          if constexpr (kNet) {
-            const float u0 = rng.next_float(), u1 = rng.next_float(), u2 = rng.next_float();
-            float d[3];
-            xbg::mix_sample(lob, u0, u1, u2, d);
-            wiw = v3(d[0], d[1], d[2]);
-          } else {
-            const float u0 = rng.next_float(), u1 = rng.next_float();
-            wiw = sky_sample(sc.sky_cdf, u0, u1);
+          if (!proposed) {
+            if (!sample_direction<kAllKinds>(wo_l, mat, fo, rng, s, lobe, scale)) break;
+            wiw = onb.to_world(s.wi);
           }
-          s.wi = onb.to_local(wiw);
-          s.delta = false;
-          if (!bsdf_lobe_for_direction(wo_l, s.wi, mat, rng.next_float(), s.f, s.pdf, pb)) break;
+        }
+        MfrHalf h{0.f, 0.f, 0.f, 0.f, 0.f};
+        if (lobe == kLobeMfr || (!nee && guided && guided_needs_mfr(mat))) h = mfr_half(wo_l, s.wi, mat);
+        if (lobe == kLobeMfr) s.pdf = h.pdf;
+        if (!nee && guided) {
+          pb = guided_density(s.wi, mat, h);
+          if (proposed && !guided_lobe(s.wi, mat, u_lobe, h, pb, lobe, s)) break;
+        }
+        if (lobe == kLobeMfr) s.f = mfr_eval(wo_l, s.wi, mat, h);
+        if (lobe == kLobeMft) mft_eval_pdf(wo_l, s.wi, mat, s.f, s.pdf);
+        if (nee) {
+          nee_combine<kAllKinds>(s.wi, mat, fo, s.f, s.pdf);
+          const float mis = pass == PASS_SUN && sc.sun_nee ? 1.f : mis_power2(nl.pdf, s.pdf);   // as in shade_kernel
+          if (pass == PASS_AREA && !(mis > 0.0f && nl.pdf > 1e-12f)) break;
+          const V3 org = offset_origin(fh.pos, fh.geo_normal, nl.wi, kShadowEps);
+          const V3 c = (tp * ratio) * s.f * s.wi.z * (nl.emission / nl.pdf) * mis;
+          q_o = make_float4(org.x, org.y, org.z, nl.tmax);
+          q_d = make_float4(nl.wi.x, nl.wi.y, nl.wi.z, __int_as_float(pid));
+          q_c = make_float4(c.x, c.y, c.z, 0.f);
         } else {
-          if (!bsdf_sample(wo_l, mat, rng, s)) break;
-          wiw = onb.to_world(s.wi);
-          pb = bsdf_density(wo_l, s.wi, mat);
+          if (lobe != kLobeNone && s.pdf < 1e-8f) break;
+          if (!s.delta) s.pdf *= scale;
+          n_ratio = ratio;
+          if (guided) {
+            const float q = kNet ? xbg::mix_pdf(lob, wiw.x, wiw.y, wiw.z) : sky_pdf(sc.sky_cdf, wiw);
+            const float pm = ap * q + (1.f - ap) * pb;
+            if (!(pm > 0.f)) break;
+            n_ratio = ratio * (pb / pm);
+            tb = tp * ratio;
+            emit_rec = training && (pid % g.rec_stride) == 0;
+          }
+          // cpu_tiled.cpp:197-216
+          if (s.delta) {
+            tp = tp * s.f;
+          } else {
+            const float ci = fabsf(s.wi.z);
+            if (s.pdf < 1e-8f || ci < 1e-8f) { emit_rec = false; break; }
+            tp = tp * (s.f * ci / s.pdf);
+          }
+          const V3 org = offset_origin(fh.pos, fh.geo_normal, wiw, kRayEps);
+          q_o = make_float4(org.x, org.y, org.z, kRayEps);
+          q_d = make_float4(wiw.x, wiw.y, wiw.z, kInf);
+          q_c = make_float4(tp.x, tp.y, tp.z, s.delta ? -1.f : s.pdf);
         }
-        const float q = kNet ? xbg::mix_pdf(lob, wiw.x, wiw.y, wiw.z) : sky_pdf(sc.sky_cdf, wiw);
-        const float pm = ap * q + (1.f - ap) * pb;
-        if (!(pm > 0.f)) break;
-        n_ratio = ratio * (pb / pm);
-        if (training && (pid % g.rec_stride) == 0) {
-          const V3 tb = tp * ratio;   // actual throughput before the vertex's scattering
-          rec[0] = make_float4(feat[0], feat[1], feat[2], feat[3]);
-          rec[1] = make_float4(feat[4], feat[5], feat[6], feat[7]);
-          rec[2] = make_float4(feat[8], wiw.x, wiw.y, wiw.z);
-          rec[3] = make_float4(0.f, __int_as_float(pid), tb.x, tb.y);
-          rec[4] = make_float4(tb.z, kNaN, kNaN, kNaN);   // baseline: set by the next bounce
-          rec[5] = make_float4(pb, 0.f, 0.f, 0.f);
-          emit_rec = true;
+        emit = true;
+      } while (false);
+      if (pass != PASS_NEXT) {
+        const int k = pass == PASS_AREA ? 0 : 1;
+        const int idx = warp_append(a.cnt + (k == 0 ? CNT_SH_AREA : CNT_SH_SUN), emit, a.capacity, a.stats + STAT_OVERFLOW);
+        if (idx >= 0) { a.sh_o[k][idx] = q_o; a.sh_d[k][idx] = q_d; a.sh_c[k][idx] = q_c; }
+        continue;
+      }
+      if constexpr (!kNet) {
+        const int gi = warp_append(a.cnt + CNT_GUIDE, emit_defer, a.capacity, a.stats + STAT_OVERFLOW);
+        if (gi >= 0) {
+          g.gq[0][gi] = make_float4(fh.pos.x, fh.pos.y, fh.pos.z, __int_as_float(fh.mat_id));
+          g.gq[1][gi] = make_float4(fh.normal.x, fh.normal.y, fh.normal.z, __int_as_float(pid));
+          g.gq[2][gi] = make_float4(fh.geo_normal.x, fh.geo_normal.y, fh.geo_normal.z, ratio);
+          g.gq[3][gi] = make_float4(wo.x, wo.y, wo.z, 0.f);
+          g.gq[4][gi] = make_float4(tp.x, tp.y, tp.z, 0.f);
+          g.gq_rng[gi] = rng.state;
         }
       }
-      // cpu_tiled.cpp:197-216
-      if (s.delta) {
-        tp = tp * s.f;
-      } else {
-        const float ci = fabsf(s.wi.z);
-        if (s.pdf < 1e-8f || ci < 1e-8f) { emit_rec = false; break; }
-        tp = tp * (s.f * ci / s.pdf);
+      int ridx = -1;
+      if (training) {
+        ridx = warp_append(g.rec_count, emit_rec, g.rec_cap, a.stats + STAT_REC_DROPPED);
+        if (ridx >= 0) write_record(g.recs, ridx, feat, v3(q_d.x, q_d.y, q_d.z), pid, tb, pb);
       }
-      const V3 org = offset_origin(fh.pos, fh.geo_normal, wiw, kRayEps);
-      n_o = make_float4(org.x, org.y, org.z, kRayEps);
-      n_d = make_float4(wiw.x, wiw.y, wiw.z, kInf);
-      n_tp = make_float4(tp.x, tp.y, tp.z, s.delta ? -1.f : s.pdf);
-      n_rng = rng.state;
-      emit_next = true;
-    } while (false);
-    if (!emit_next) emit_rec = false;
-    if constexpr (!kNet) {
-      const int gi = warp_append(a.cnt + CNT_GUIDE, emit_defer, a.capacity, a.stats + STAT_OVERFLOW);
-      if (gi >= 0) {
-        for (int k = 0; k < 5; ++k) g.gq[k][gi] = dq[k];
-        g.gq_rng[gi] = n_rng;
+      const int idx = warp_append(a.cnt_next + CNT_RAYS, emit, a.capacity, a.stats + STAT_OVERFLOW);
+      if (idx >= 0) {
+        a.nray_o[idx] = q_o; a.nray_d[idx] = q_d; a.ntp[idx] = q_c;
+        a.nrng[idx] = rng.state;
+        a.npath[idx] = pid;
+        g.ratio_out[idx] = n_ratio;
+        if (g.rec_out) g.rec_out[idx] = ridx;
       }
     }
-    int ridx = -1;
-    if (training) {
-      ridx = warp_append(g.rec_count, emit_rec, g.rec_cap, a.stats + STAT_REC_DROPPED);
-      if (ridx >= 0) {
-        float4* R = reinterpret_cast<float4*>(g.recs + (size_t)ridx * xbg::kRecFloats);
-        for (int i = 0; i < 6; ++i) R[i] = rec[i];
-      }
-    }
-    int idx = warp_append(a.cnt_next + CNT_RAYS, emit_next, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) {
-      a.nray_o[idx] = n_o; a.nray_d[idx] = n_d; a.ntp[idx] = n_tp; a.nrng[idx] = n_rng;
-      a.npath[idx] = pid;
-      g.ratio_out[idx] = n_ratio;
-      if (g.rec_out) g.rec_out[idx] = ridx;
-    }
-    idx = warp_append(a.cnt + CNT_SH_AREA, emit_area, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) { a.sh_o[0][idx] = a_o; a.sh_d[0][idx] = a_d; a.sh_c[0][idx] = a_c; }
-    idx = warp_append(a.cnt + CNT_SH_SUN, emit_sun, a.capacity, a.stats + STAT_OVERFLOW);
-    if (idx >= 0) { a.sh_o[1][idx] = s_o; a.sh_d[1][idx] = s_d; a.sh_c[1][idx] = s_c; }
   }
   if constexpr (kNet) xbg::mma_teardown(m.tmem);
 }
@@ -943,11 +914,10 @@ __global__ void __launch_bounds__(128, 4) guide_sample_kernel(ShadeArgs a, Guide
       xbg::raw_to_lobes<true>(raw, lob);
       alpha = g.alpha >= 0.f ? g.alpha : xbg::selection<true>(raw);
     }
-    bool emit_next = false, emit_rec = false;
+    bool emit = false, emit_rec = false;
     float4 n_o, n_d, n_tp;
-    float4 rec[6];
-    uint64_t n_rng = 0;
-    float n_ratio = 1.f;
+    float n_ratio = 1.f, pb = 0.f;
+    V3 tb = v3s(0.f);   // actual throughput before the vertex's scattering
     const int32_t pid = __float_as_int(q[1].w);
     if (valid) do {
       const DevMaterial& mat = sc.mats[__float_as_int(q[0].w)];
@@ -958,57 +928,56 @@ __global__ void __launch_bounds__(128, 4) guide_sample_kernel(ShadeArgs a, Guide
       const V3 wo_l = onb.to_local(v3(q[3].x, q[3].y, q[3].z));
       BsdfSample s;
       V3 wiw;
-      float pb;
+      int lobe = kLobeNone;
+      float scale = 1.f, u_lobe = 0.f;
       const float ap = capped_selection(alpha, ratio, g.ratio_cap);
-      if (rng.next_float() < ap) {
+      const bool proposed = rng.next_float() < ap;
+      if (proposed) {
         const float u0 = rng.next_float(), u1 = rng.next_float(), u2 = rng.next_float();
         float d[3];
         xbg::mix_sample(lob, u0, u1, u2, d);
         wiw = v3(d[0], d[1], d[2]);
         s.wi = onb.to_local(wiw);
-        s.delta = false;
-        if (!bsdf_lobe_for_direction(wo_l, s.wi, mat, rng.next_float(), s.f, s.pdf, pb)) break;
+        u_lobe = rng.next_float();
       } else {
-        if (!bsdf_sample(wo_l, mat, rng, s)) break;
+        if (!sample_direction<kGuidedKinds>(wo_l, mat, 0.f, rng, s, lobe, scale)) break;
         wiw = onb.to_world(s.wi);
-        pb = bsdf_density(wo_l, s.wi, mat);
       }
+      MfrHalf h{0.f, 0.f, 0.f, 0.f, 0.f};
+      if (guided_needs_mfr(mat)) h = mfr_half(wo_l, s.wi, mat);
+      pb = guided_density(s.wi, mat, h);
+      if (proposed) {
+        if (!guided_lobe(s.wi, mat, u_lobe, h, pb, lobe, s)) break;
+      } else {
+        if (lobe == kLobeMfr) s.pdf = h.pdf;
+        if (s.pdf < 1e-8f) break;
+        s.pdf *= scale;
+      }
+      if (lobe == kLobeMfr) s.f = mfr_eval(wo_l, s.wi, mat, h);
       const float pm = ap * xbg::mix_pdf(lob, wiw.x, wiw.y, wiw.z) + (1.f - ap) * pb;
       if (!(pm > 0.f)) break;
       n_ratio = ratio * (pb / pm);
-      if (training && (pid % g.rec_stride) == 0) {
-        const V3 tb = tp * ratio;   // actual throughput before the vertex's scattering
-        rec[0] = make_float4(feat[0], feat[1], feat[2], feat[3]);
-        rec[1] = make_float4(feat[4], feat[5], feat[6], feat[7]);
-        rec[2] = make_float4(feat[8], wiw.x, wiw.y, wiw.z);
-        rec[3] = make_float4(0.f, __int_as_float(pid), tb.x, tb.y);
-        rec[4] = make_float4(tb.z, kNaN, kNaN, kNaN);   // baseline: set by the next bounce
-        rec[5] = make_float4(pb, 0.f, 0.f, 0.f);
-        emit_rec = true;
-      }
+      tb = tp * ratio;
       // cpu_tiled.cpp:197-216 (the guided lobes are never delta)
       const float ci = fabsf(s.wi.z);
-      if (s.pdf < 1e-8f || ci < 1e-8f) { emit_rec = false; break; }
+      if (s.pdf < 1e-8f || ci < 1e-8f) break;
       tp = tp * (s.f * ci / s.pdf);
       const V3 org = offset_origin(pos, gn, wiw, kRayEps);
       n_o = make_float4(org.x, org.y, org.z, kRayEps);
       n_d = make_float4(wiw.x, wiw.y, wiw.z, kInf);
       n_tp = make_float4(tp.x, tp.y, tp.z, s.pdf);
-      n_rng = rng.state;
-      emit_next = true;
+      emit_rec = training && (pid % g.rec_stride) == 0;
+      emit = true;
     } while (false);
-    if (!emit_next) emit_rec = false;
     int ridx = -1;
     if (training) {
       ridx = warp_append(g.rec_count, emit_rec, g.rec_cap, a.stats + STAT_REC_DROPPED);
-      if (ridx >= 0) {
-        float4* R = reinterpret_cast<float4*>(g.recs + (size_t)ridx * xbg::kRecFloats);
-        for (int i = 0; i < 6; ++i) R[i] = rec[i];
-      }
+      if (ridx >= 0) write_record(g.recs, ridx, feat, v3(n_d.x, n_d.y, n_d.z), pid, tb, pb);
     }
-    const int idx = warp_append(a.cnt_next + CNT_RAYS, emit_next, a.capacity, a.stats + STAT_OVERFLOW);
+    const int idx = warp_append(a.cnt_next + CNT_RAYS, emit, a.capacity, a.stats + STAT_OVERFLOW);
     if (idx >= 0) {
-      a.nray_o[idx] = n_o; a.nray_d[idx] = n_d; a.ntp[idx] = n_tp; a.nrng[idx] = n_rng;
+      a.nray_o[idx] = n_o; a.nray_d[idx] = n_d; a.ntp[idx] = n_tp;
+      a.nrng[idx] = rng.state;
       a.npath[idx] = pid;
       g.ratio_out[idx] = n_ratio;
       if (g.rec_out) g.rec_out[idx] = ridx;
