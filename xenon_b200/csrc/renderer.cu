@@ -296,14 +296,14 @@ __global__ void raygen_kernel(CamDev cam, int W, int H, int spp_first, int64_t p
 
 // ── extend: closest hit of the bounce's ray queue (trace_persistent.cuh) ──────────
 template <bool kCount, int kSh>
-__global__ void __launch_bounds__(128) extend_persistent_kernel(DevScene sc, TraceQueue q, int refill) {
-  QueueIO io{q, *q.count};
+__global__ void __launch_bounds__(128, 7) extend_persistent_kernel(DevScene sc, TraceQueue q, int refill, int warps) {
+  QueueIO io(q, warps);
   trace_persistent<false, kCount, kSh>(sc, io, refill, false);
 }
 // ── shadow: any hit; unoccluded items add their contribution ──────────────────
 template <bool kCount, int kSh>
-__global__ void __launch_bounds__(128) shadow_persistent_kernel(DevScene sc, TraceQueue q, int refill) {
-  QueueIO io{q, *q.count};
+__global__ void __launch_bounds__(128) shadow_persistent_kernel(DevScene sc, TraceQueue q, int refill, int warps) {
+  QueueIO io(q, warps);
   trace_persistent<true, kCount, kSh>(sc, io, refill, q.far_first != 0);
 }
 
@@ -1163,6 +1163,7 @@ struct ApiIO {
   bool wide;
   int next, stop;
   __device__ __forceinline__ int end() const { return stop; }
+  __device__ __forceinline__ int lanes() const { return 32; }
   __device__ __forceinline__ int grab(int, int, int k) {
     const int b = next;
     next += k;
@@ -1671,7 +1672,8 @@ void launch_extend_k(xb_renderer* r, const LaneRef& L, int d, bool count) {
   TraceQueue tq{w.ray_o[q], w.ray_d[q], cd_ + CNT_RAYS, cd_ + CNT_FETCH_EXT, w.hit, w.hit_inst,
                 nullptr, nullptr, r->stats, 0};
   auto kern = count ? extend_persistent_kernel<true, kSh> : extend_persistent_kernel<false, kSh>;
-  kern<<<per_thread ? r->grid_ext : r->grid_pext, 128, smem, L.s>>>(r->scene, tq, per_thread ? 32 : r->refill);
+  kern<<<per_thread ? r->grid_ext : r->grid_pext, 128, smem, L.s>>>(r->scene, tq, per_thread ? 32 : r->refill,
+                                                                   r->num_sms * r->occ_pext * 4);
 }
 
 void launch_extend(xb_renderer* r, const LaneRef& L, int d, bool count) {
@@ -1690,7 +1692,8 @@ void launch_shadow_k(xb_renderer* r, const LaneRef& L, int d, int k, bool count,
                 cd_ + (k ? CNT_FETCH_SH_SUN : CNT_FETCH_SH_AREA), nullptr, nullptr, w.sh_c[k], w.L,
                 r->stats, r->tune.shadow_order == 2};
   auto kern = count ? shadow_persistent_kernel<true, kSh> : shadow_persistent_kernel<false, kSh>;
-  kern<<<per_thread ? r->grid_shadow : r->grid_pshadow, 128, smem, s>>>(r->scene, tq, per_thread ? 32 : r->refill);
+  kern<<<per_thread ? r->grid_shadow : r->grid_pshadow, 128, smem, s>>>(r->scene, tq, per_thread ? 32 : r->refill,
+                                                                       r->num_sms * r->occ_pshadow * 4);
 }
 
 void launch_shadows(xb_renderer* r, const LaneRef& L, int d, bool count, cudaStream_t s) {
@@ -3023,7 +3026,12 @@ int xb_trace_rays_device(xb_renderer* r, const xb_ray* rays, int64_t n, xb_hit* 
   const bool wide = aligned16(rays, hits);
   for (int64_t at = 0; at < n; at += kMaxLaunchRays) {
     const int m = (int)std::min(n - at, kMaxLaunchRays);
-    const int grid = (int)std::min<int64_t>(((int64_t)m + 127) / 128, (int64_t)r->num_sms * r->occ_api[any]);
+    // a batch that would put fewer than 2 blocks on an SM is spread over 4, 8 rays to a warp at
+    // least (1000 hemisphere rays on 261 instances: closest 116 -> 92 us, any 93 -> 80; 20000: 152
+    // -> 132, 124 -> 111); beyond, full warps are faster (65536 on one mesh: 113 us, spread 134)
+    const int64_t full = ((int64_t)m + 127) / 128, sms = r->num_sms;
+    const int64_t blocks = full >= 2 * sms ? full : std::max(full, std::min(((int64_t)m + 31) / 32, 4 * sms));
+    const int grid = (int)std::min(blocks, sms * r->occ_api[any]);
     auto kern = any ? trace_api_persistent_kernel<true> : trace_api_persistent_kernel<false>;
     kern<<<grid, 128, 0, s>>>(r->scene, rays + at, m, hits + at, r->stats, refill, wide);
   }
