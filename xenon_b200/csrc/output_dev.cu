@@ -127,40 +127,45 @@ __global__ void digit_hist_kernel(const uint32_t* __restrict__ rel, int64_t n, i
   }
 }
 
-struct Scratch {
-  void* p = nullptr;
-  ~Scratch() { if (p) cudaFree(p); }
-};
+int stage_blocks(int64_t n, int num_sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, (int64_t)num_sms * 8));
+}
+size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
+constexpr size_t kHistBytes = 65536 * 4;
 
 }  // namespace
 
-int device_output_stage(const float* d_img, int W, int H, int num_sms, cudaStream_t s, uint8_t* rgb8,
+size_t output_stage_bytes(int W, int H, int num_sms) {
+  const size_t n = (size_t)W * H;
+  return up256(3 * n) + up256(8 * n) + up256((size_t)stage_blocks((int64_t)n, num_sms) * 16) + 256 + kHistBytes;
+}
+
+int device_output_stage(const float* d_img, int W, int H, int num_sms, cudaStream_t s, void* ws, uint8_t* rgb8,
                         xb_noise_stats* out) {
   const int64_t n = (int64_t)W * H;
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, (int64_t)num_sms * 8));
+  const int blocks = stage_blocks(n, num_sms);
   auto ck = [](cudaError_t e) { return e == cudaSuccess; };
+  char* base = static_cast<char*>(ws);
   if (rgb8) {
-    Scratch d8;
-    if (!ck(cudaMalloc(&d8.p, (size_t)n * 3))) return fail(XB_E_OOM, "output stage: out of device memory");
-    rgb8_kernel<<<blocks, kThreads, 0, s>>>(d_img, W, H, static_cast<uint8_t*>(d8.p));
-    if (!ck(cudaMemcpyAsync(rgb8, d8.p, (size_t)n * 3, cudaMemcpyDeviceToHost, s)) || !ck(cudaStreamSynchronize(s)))
+    uint8_t* d8 = reinterpret_cast<uint8_t*>(base);
+    rgb8_kernel<<<blocks, kThreads, 0, s>>>(d_img, W, H, d8);
+    if (!ck(cudaMemcpyAsync(rgb8, d8, (size_t)n * 3, cudaMemcpyDeviceToHost, s)) || (!out && !ck(cudaStreamSynchronize(s))))
       return fail(XB_E_CUDA, "output stage: %s", cudaGetErrorString(cudaGetLastError()));
   }
+  base += up256(3 * (size_t)n);
   if (!out) return XB_OK;
   std::memset(out, 0, sizeof(*out));
-  if (W <= 2 || H <= 2) return XB_OK;   // no interior pixel
+  if (W <= 2 || H <= 2)   // no interior pixel
+    return ck(cudaStreamSynchronize(s)) ? XB_OK : fail(XB_E_CUDA, "output stage: %s", cudaGetErrorString(cudaGetLastError()));
   out->total_interior_pixel_count = (W - 2) * (H - 2);
-  // scratch: luminance and residual bits (n each), block sums, count and maximum, one histogram
-  const size_t b_lum = (size_t)n * 4, b_part = (size_t)blocks * 2 * 8, b_hist = 65536 * 4;
-  Scratch sc;
-  if (!ck(cudaMalloc(&sc.p, 2 * b_lum + b_part + 256 + b_hist))) return fail(XB_E_OOM, "output stage: out of device memory");
-  char* base = static_cast<char*>(sc.p);
+  // luminance and residual bits (n each), block sums, count and maximum, one histogram
+  const size_t b_part = (size_t)blocks * 16, b_hist = kHistBytes;
   float* lum = reinterpret_cast<float*>(base);
-  uint32_t* rel = reinterpret_cast<uint32_t*>(base + b_lum);
-  double* part = reinterpret_cast<double*>(base + 2 * b_lum);
-  int* cnt = reinterpret_cast<int*>(base + 2 * b_lum + b_part);
+  uint32_t* rel = reinterpret_cast<uint32_t*>(lum + n);
+  double* part = reinterpret_cast<double*>(base + up256(8 * (size_t)n));
+  int* cnt = reinterpret_cast<int*>(reinterpret_cast<char*>(part) + up256(b_part));
   unsigned int* amax = reinterpret_cast<unsigned int*>(cnt + 1);
-  unsigned int* hist = reinterpret_cast<unsigned int*>(base + 2 * b_lum + b_part + 256);
+  unsigned int* hist = reinterpret_cast<unsigned int*>(cnt + 64);
   std::vector<double> hp((size_t)blocks * 2);
   lum_kernel<<<blocks, kThreads, 0, s>>>(d_img, n, lum, part);
   if (!ck(cudaMemcpyAsync(hp.data(), part, (size_t)blocks * 8, cudaMemcpyDeviceToHost, s)) || !ck(cudaStreamSynchronize(s)))
