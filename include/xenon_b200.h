@@ -318,7 +318,7 @@ int  xb_upload_scene(xb_renderer *r, const xb_scene_view *view);
  * float[3 * nv] (nv = the mesh's vertex count in the uploaded view); normals: the same, or NULL
  * to keep the uploaded ones. Meshes that carry area lights are refused (XB_E_UNSUPPORTED: their
  * emitter geometry is built on the host at upload; refit the host scene and upload again).
- * Synchronises the render stream; captured bounce graphs are rebuilt on the next render. The
+ * Synchronises the render stream. The
  * arrays are rewritten in place, so ray queries issued on caller streams (xb_trace_rays_device,
  * xb_trace_rays_noalloc) must have finished before this call. If the uploaded BLAS turns out to
  * be malformed (XB_E_INVALID), some of it has already been rewritten: the renderer then holds no

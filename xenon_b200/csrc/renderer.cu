@@ -2105,17 +2105,28 @@ __global__ void flip_rows_f64_kernel(const double* __restrict__ src, double* __r
 
 // ── BLAS refit (xb_refit_mesh): one mesh's triangles and node boxes, topology kept ──────────
 // The passes are refit_kernels.h's, which the host refit (xb_scene_refit_mesh) runs as loops.
+__global__ void refit_finite_kernel(xb::RefitArgs a, const float* normals) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < 3 * (int64_t)a.num_verts && (!isfinite(a.pos[i]) || (normals && !isfinite(normals[i])))) atomicExch(a.status + 1, 1);
+}
+__global__ void refit_normals_kernel(xb::RefitArgs a, const float* normals, float* nx, float* ny, float* nz) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.num_verts || a.status[1] != 0) return;
+  nx[a.vtx_offset + i] = normals[3 * (int64_t)i];
+  ny[a.vtx_offset + i] = normals[3 * (int64_t)i + 1];
+  nz[a.vtx_offset + i] = normals[3 * (int64_t)i + 2];
+}
 __global__ void refit_tris_kernel(xb::RefitArgs a) {
   const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < a.num_tris) xb::refit_tris_at(a, s);
+  if (s < a.num_tris && a.status[1] == 0) xb::refit_tris_at(a, s);
 }
 __global__ void refit_parents_kernel(xb::RefitArgs a) {
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < a.num_nodes) xb::refit_parents_at(a, i);
+  if (i < a.num_nodes && a.status[1] == 0) xb::refit_parents_at(a, i);
 }
 __global__ void refit_nodes_kernel(xb::RefitArgs a) {
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < a.num_nodes) xb::refit_nodes_at(a, i);
+  if (i < a.num_nodes && a.status[1] == 0) xb::refit_nodes_at(a, i);
 }
 
 }  // namespace
@@ -2495,7 +2506,6 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.num_lights = v->num_lights;
   sc.num_suns = v->num_suns;
   sc.num_tlas_nodes = v->num_tlas_nodes;
-  if (!tlas.empty()) { sc.root_a = tlas[0]; sc.root_b = tlas[1]; }
   r->tlas_cap = tlas_cap;
   r->big_leaves = (int64_t)big_leaves.size();
   r->loose_blas = loose;
@@ -2530,16 +2540,20 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   if (normals && !ml.has_normals)
     return set_err(r, XB_E_INVALID, "xb_refit_mesh: mesh %d was uploaded without normals", mesh);
   const int64_t nv = ml.num_verts;
-  for (int64_t i = 0; i < 3 * nv; ++i)
-    if (!std::isfinite(positions[i]) || (normals && !std::isfinite(normals[i])))
-      return set_err(r, XB_E_INVALID, "xb_refit_mesh: non-finite value at %lld", (long long)i);
-  if (ml.num_nodes == 0 || ml.num_tris == 0) return XB_OK;
+  if (ml.num_nodes == 0 || ml.num_tris == 0) {
+    for (int64_t i = 0; i < 3 * nv; ++i)
+      if (!std::isfinite(positions[i]) || (normals && !std::isfinite(normals[i])))
+        return set_err(r, XB_E_INVALID, "xb_refit_mesh: non-finite value at %lld", (long long)i);
+    return XB_OK;
+  }
   sync_lanes(r);                          // no wave may read the scene while it changes
   CK(cudaStreamSynchronize(r->stream));
   // scratch: positions, normals, parents, arrival counts, status (256-byte aligned pieces)
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t b_pos = up(12 * (size_t)nv), b_nodes = up(4 * (size_t)ml.num_nodes);
   const size_t need = b_pos * (normals ? 2 : 1) + 2 * b_nodes + 256;
+  DevScene before;
+  std::memcpy(&before, &r->scene, sizeof(before));
   if (need > r->refit_bytes) {
     if (r->refit_mem) CK(cudaFree(r->refit_mem));
     r->refit_mem = nullptr;
@@ -2558,7 +2572,7 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   char* rest = base + b_pos * (normals ? 2 : 1);
   a.parent = reinterpret_cast<int32_t*>(rest);
   a.arrivals = reinterpret_cast<uint32_t*>(rest + b_nodes);
-  a.status = reinterpret_cast<int32_t*>(rest + 2 * b_nodes);
+  a.status = reinterpret_cast<int32_t*>(rest + 2 * b_nodes);   // and, after it, the finite check's
   a.big_leaves = reinterpret_cast<const uint32_t*>(r->scene.big_leaves);
   a.child_mask = kLeafEntry - 1u;
   a.big_count = kEntryEscape;
@@ -2570,29 +2584,29 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   a.tri_offset = ml.tri_offset;
   a.vtx_offset = ml.vtx_offset;
   cudaStream_t s = r->stream;
+  CK(cudaMemsetAsync(a.status, 0, 2 * sizeof(int32_t), s));
   CK(cudaMemcpyAsync(pos_dev, positions, 12 * (size_t)nv, cudaMemcpyHostToDevice, s));
-  if (normals) {
-    // the device keeps normals as three arrays over all vertices: one copy per component
-    CK(cudaMemcpyAsync(nrm, normals, 12 * (size_t)nv, cudaMemcpyHostToDevice, s));
-    float* dst[3] = {const_cast<float*>(r->scene.nx), const_cast<float*>(r->scene.ny),
-                     const_cast<float*>(r->scene.nz)};
-    for (int k = 0; k < 3; ++k)
-      CK(cudaMemcpy2DAsync(dst[k] + ml.vtx_offset, sizeof(float), nrm + k, 3 * sizeof(float), sizeof(float),
-                           (size_t)nv, cudaMemcpyDeviceToDevice, s));
-  }
+  if (normals) CK(cudaMemcpyAsync(nrm, normals, 12 * (size_t)nv, cudaMemcpyHostToDevice, s));
+  // a non-finite value: the kernels after this one leave the scene as it is
+  refit_finite_kernel<<<(int)((3 * nv + 255) / 256), 256, 0, s>>>(a, nrm);
+  if (normals)   // the device keeps normals as three arrays over all vertices
+    refit_normals_kernel<<<(int)((nv + 255) / 256), 256, 0, s>>>(a, nrm, const_cast<float*>(r->scene.nx),
+                                                                 const_cast<float*>(r->scene.ny),
+                                                                 const_cast<float*>(r->scene.nz));
   CK(cudaMemsetAsync(a.parent, 0xff, 4 * (size_t)ml.num_nodes, s));
-  CK(cudaMemsetAsync(a.status, 0, sizeof(int32_t), s));
   refit_tris_kernel<<<(ml.num_tris + 255) / 256, 256, 0, s>>>(a);
   refit_parents_kernel<<<(ml.num_nodes + 255) / 256, 256, 0, s>>>(a);
   refit_nodes_kernel<<<(ml.num_nodes + 255) / 256, 256, 0, s>>>(a);
   CK(cudaGetLastError());
-  int32_t status = 0;
-  float4 root[2];
-  CK(cudaMemcpyAsync(&status, a.status, sizeof(status), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(root, r->scene.nodes + 2 * ml.node_base, sizeof(root), cudaMemcpyDeviceToHost, s));
+  int32_t* const st = reinterpret_cast<int32_t*>(r->host_stage);          // status and the finite check's
+  float4* const root = reinterpret_cast<float4*>(r->host_stage + 256);
+  CK(cudaMemcpyAsync(st, a.status, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(root, r->scene.nodes + 2 * ml.node_base, 2 * sizeof(float4), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  drop_graphs(r);
+  if (st[1] != 0) return set_err(r, XB_E_INVALID, "xb_refit_mesh: non-finite value in the positions or normals");
+  const int32_t status = st[0];
   if (status != 0) {
+    drop_graphs(r);
     // the triangles and some boxes are rewritten already: no render may trace this scene
     r->has_scene = false;
     return set_err(r, XB_E_INVALID, "xb_refit_mesh: mesh %d's BLAS is malformed (%s); upload the scene again",
@@ -2624,8 +2638,6 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
     return set_err(r, XB_E_UNSUPPORTED, "xb_refit_mesh: the rebuilt TLAS does not fit the uploaded scene's");
   if (!tlas.empty()) {
     CK(cudaMemcpy(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    sc.root_a = tlas[0];
-    sc.root_b = tlas[1];
   }
   sc.loose_boxes = r->loose_blas || loose_tlas;
   if (!order.empty()) {
@@ -2634,12 +2646,16 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
                   cudaMemcpyHostToDevice));
   }
   sc.num_tlas_nodes = (int32_t)nodes.size();
+  bool moved = false;
   if (!nodes.empty()) {
     for (int k = 0; k < 3; ++k) {
+      moved = moved || r->scene_lo[k] != nodes[0].mn[k] || r->scene_hi[k] != nodes[0].mx[k];
       r->scene_lo[k] = nodes[0].mn[k];
       r->scene_hi[k] = nodes[0].mx[k];
     }
   }
+  // the captured bounce loops hold the scene's pointers and counts, and guided ones its bounds
+  if (std::memcmp(&before, &sc, sizeof(sc)) != 0 || (r->guide && moved)) drop_graphs(r);
   return XB_OK;
 }
 

@@ -269,10 +269,12 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, IO& io, int
           occluded = false;
           if (sc.num_tlas_nodes > 0) {
             if (kCount) cnt.tlas++;
+            float4 root_a, root_b;
+            ldg8(sc.nodes, root_a, root_b);
             float tn;
-            if (odd ? aabb_fast(sc.root_a, sc.root_b, winv, wo, wd, tmin, t_best, tn)
-                    : sr.slab(sc.root_a, sc.root_b, tmin, t_best, tn)) {
-              cur = __float_as_uint(sc.root_b.z);
+            if (odd ? aabb_fast(root_a, root_b, winv, wo, wd, tmin, t_best, tn)
+                    : sr.slab(root_a, root_b, tmin, t_best, tn)) {
+              cur = __float_as_uint(root_b.z);
               if (cur < kLeafEntry) cur >>= 1;
             }
           }
