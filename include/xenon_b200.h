@@ -428,8 +428,10 @@ typedef struct xb_tuning {
   int32_t shadow_blocks_per_sm;         /* and shade kernels (1-64); for the persistent ones */
   int32_t shade_blocks_per_sm;          /* bounded by the blocks that fit on an SM at once */
   int32_t wave_paths;                   /* paths in flight per wave (reallocates queues) */
-  int32_t shadow_order;                 /* shadow rays: 1 nearer child first, 2 farther first
-                                           (the occlusion answer does not depend on it) */
+  int32_t shadow_order;                 /* shadow rays: 1 nearer child first, 2 (default) farther
+                                           first: a ray starts on a surface, among boxes that do not
+                                           occlude it (1-8 % per sample on every scene measured;
+                                           the occlusion answer does not depend on it) */
   int32_t overlap;                      /* 1: a bounce's shadow rays run on a second stream,
                                            concurrently with the next bounce's closest hits;
                                            2: one stream */

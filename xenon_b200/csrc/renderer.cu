@@ -1565,7 +1565,7 @@ int apply_tuning(xb_renderer* r, const xb_tuning& t) {
   c.shadow_blocks_per_sm = std::min(64, pick(t.shadow_blocks_per_sm, c.shadow_blocks_per_sm, 64));
   c.shade_blocks_per_sm = std::min(64, pick(t.shade_blocks_per_sm, c.shade_blocks_per_sm, 64));
   c.wave_paths = pick(t.wave_paths, c.wave_paths, 1 << 21);
-  c.shadow_order = pick(t.shadow_order, c.shadow_order, 1);
+  c.shadow_order = pick(t.shadow_order, c.shadow_order, 2);
   c.overlap = pick(t.overlap, c.overlap, 1);
   c.waves = std::min(kMaxLanes, pick(t.waves, c.waves, 2));
   c.lane_stagger = std::min(kMaxDepth, pick(t.lane_stagger, c.lane_stagger, 1));
@@ -2149,9 +2149,8 @@ int xb_create(const xb_config* cfg, xb_renderer** out) {
   r->max_bounces = std::min(cfg->max_bounces, kMaxDepth);
   auto bail = [&](int code) { xb_destroy(r); return code; };
   if (cudaSetDevice(cfg->device) != cudaSuccess) return bail(xb::fail(XB_E_CUDA, "cudaSetDevice failed"));
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, cfg->device) != cudaSuccess) return bail(xb::fail(XB_E_CUDA, "cudaGetDeviceProperties failed"));
-  r->num_sms = prop.multiProcessorCount;
+  if (cudaDeviceGetAttribute(&r->num_sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
+    return bail(xb::fail(XB_E_CUDA, "cudaDeviceGetAttribute failed"));
   if (cudaStreamCreateWithFlags(&r->stream2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&r->copy_stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(xb::fail(XB_E_CUDA, "stream creation failed"));
