@@ -94,18 +94,20 @@ __device__ __forceinline__ int tile_start(int n, int batch, uint64_t seed, uint6
   return (int)(h % (uint64_t)(n - kTile + 1));
 }
 
-// Sum of the weights c over the step's batch (one block per tile, added into *csum).
+// Sum of the weights c over the batch of each step t0 + blockIdx.y (one block per tile and step,
+// added into csum[blockIdx.y]): the batches depend on the step's number alone, so one launch serves
+// all steps of a call.
 __global__ void weight_sum_kernel(const float* recs, const int32_t* rec_count, int cap, int batch, uint64_t seed,
-                                  uint64_t t, float* csum) {
+                                  uint64_t t0, float* csum) {
   __shared__ float part[4];
   const int n = min(*rec_count, cap);
-  const int start = tile_start(n, batch, seed, t, blockIdx.x);
+  const int start = tile_start(n, batch, seed, t0 + blockIdx.y, blockIdx.x);
   const int i = start + threadIdx.x;
   float c = i < n ? recs[(size_t)i * kRecFloats + 12] : 0.f;
   for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
   __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(csum, part[0] + part[1] + part[2] + part[3]);
+  if (threadIdx.x == 0) atomicAdd(csum + blockIdx.y, part[0] + part[1] + part[2] + part[3]);
 }
 
 struct TrainArgs {
@@ -174,6 +176,26 @@ __device__ __forceinline__ float output_gradient(const float* raw, const float* 
   return loss;
 }
 
+// Floats per row of the FP32 error signal in shared memory: a thread writes its row, and with 64
+// floats to a row all 32 lanes of a warp would write to one bank.
+constexpr int kDfStride = kHid + 1;
+
+// load_matrix without waiting: 16-byte asynchronous copies, complete after cp_async_wait.
+__device__ __forceinline__ void load_matrix_async(uint8_t* dst, const __nv_bfloat16* src, int rows, int K) {
+  const int chunks = K / 8;
+  for (int i = threadIdx.x; i < rows * chunks; i += blockDim.x) {
+    const int r = i / chunks, c = i % chunks;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + kmajor_offset(r, c * 8, K))),
+                 "l"(src + (size_t)r * K + c * 8)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 // This tile's weight gradient of a layer from TMEM columns [64, 128) (run_backward): thread o < O
 // adds its row dW[o][0..64) into gW with 16-byte atomics; and db[o] += sum_r delta[r][o] from the
 // FP32 error signal. Every thread takes part in the TMEM loads.
@@ -189,24 +211,31 @@ __device__ __forceinline__ void add_weight_grad(const Mma& m, const float* sDf, 
       for (int q = 0; q < 4; ++q) atomicAdd(dst + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
     }
   }
-  if (o < O) {
+  // the bias: each half of the threads sums half of the rows
+  const int ob = threadIdx.x & (kHid - 1), r0 = threadIdx.x / kHid * (kTile / 2);
+  if (ob < O) {
     float s = 0.f;
-    for (int r = 0; r < kTile; ++r) s += sDf[r * kHid + o];
-    atomicAdd(gB + o, s);
+#pragma unroll 16
+    for (int r = 0; r < kTile / 2; ++r) s += sDf[(r0 + r) * kDfStride + ob];
+    atomicAdd(gB + ob, s);
   }
 }
 
 constexpr uint32_t kBwdWeightBytes = 3 * kWBytes + kW3bBytes;
 constexpr size_t kInferSmem = kFwdWeightBytes + kTileBytes + 1024;
-constexpr size_t kTrainSmem = kFwdWeightBytes + kBwdWeightBytes + 5 * kTileBytes + kTile * kHid * 4 + 1024;
+constexpr size_t kTrainSmem = kFwdWeightBytes + kBwdWeightBytes + 5 * kTileBytes + kTile * kDfStride * 4 + 1024;
 
+// What bounds it: the serial chain of one 128-row tile per CTA (8 MMA commits with their epilogues);
+// a batch of 16384 is 128 CTAs, less than one per SM. B200, a step of that batch with its Adam launch
+// 52 -> 35 us: the padded error signal (a 32-way bank conflict before), the ReLU mask in 16-byte
+// loads, the bias sums on all threads, asynchronous weight copies, one weight-sum launch per call.
 __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sWf = smem;
   uint8_t* sWb = sWf + kFwdWeightBytes;
   uint8_t* sAct = sWb + kBwdWeightBytes;                    // a0 .. a3, one tile each
   uint8_t* sD = sAct + 4 * kTileBytes;                      // delta as the bf16 A operand
-  float* sDf = reinterpret_cast<float*>(sD + kTileBytes);   // delta in FP32, [128][64]
+  float* sDf = reinterpret_cast<float*>(sD + kTileBytes);   // delta in FP32, rows of kDfStride
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_slot;
   __shared__ float sBias[kBiasFloats];
@@ -215,9 +244,12 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
   const int start = tile_start(n, A.batch, A.seed, A.t, blockIdx.x);
   if (start >= n) return;
   const float csum = *A.csum;
-  load_forward_weights(sWf, sBias, A.wf, A.master);
-  for (int l = 0; l < 3; ++l) load_matrix(sWb + l * kWBytes, A.wb + l * kHid * kK, kHid, kK);
-  load_matrix(sWb + 3 * kWBytes, A.wb + 3 * kHid * kK, kHid, kOut);
+  // the forward weights arrive during the encoding, the backward ones during the forward pass
+  for (int l = 0; l < 4; ++l) load_matrix_async(sWf + l * kWBytes, A.wf + l * kHid * kK, l < 3 ? kHid : kOut, kK);
+  cp_async_commit();
+  for (int l = 0; l < 4; ++l) load_matrix_async(sWb + l * kWBytes, A.wb + l * kHid * kK, kHid, l < 3 ? kK : kOut);
+  cp_async_commit();
+  load_biases(sBias, A.master);
   mma_setup(&tmem_slot, &mbar, 128);
   Mma m{tmem_slot, &mbar, 0u, A.err, true};
   const bool valid = start + (int)threadIdx.x < n;
@@ -230,6 +262,7 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
     pb = R[20];
   }
   encode_row(f, sAct, threadIdx.x);
+  cp_async_wait<1>();
   for (int l = 0; l < 3 && m.ok; ++l) {
     m.sync_before();
     m.run(smem_u32(sAct + l * kTileBytes), smem_u32(sWf + l * kWBytes), kK, kHid);
@@ -247,7 +280,8 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
     const float cb = (valid && csum > 0.f) ? c / csum : 0.f;
     float g[kOut];
     loss_part = output_gradient(raw, om, cb, pb, A.alpha_fixed, g);
-    for (int i = 0; i < kOut; ++i) sDf[threadIdx.x * kHid + i] = g[i];
+#pragma unroll
+    for (int i = 0; i < kOut; ++i) sDf[threadIdx.x * kDfStride + i] = g[i];
     for (int k0 = 0; k0 < kOut; k0 += 8) store8_bf16(sD, threadIdx.x, k0, kOut, g + k0);
   }
   for (int off = 16; off > 0; off >>= 1) loss_part += __shfl_xor_sync(0xffffffffu, loss_part, off);
@@ -256,6 +290,7 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
   if (threadIdx.x == 0) atomicAdd(A.loss, sLoss[0] + sLoss[1] + sLoss[2] + sLoss[3]);
   // backward: dW_l = delta_l^T a_l and delta_{l-1} = (delta_l W_l) o [a_l > 0], both on the tensor
   // cores in one commit (run_backward)
+  cp_async_wait<0>();
   for (int l = 3; l >= 0 && m.ok; --l) {
     const int O = l == 3 ? kOut : kHid;
     m.sync_before();
@@ -267,10 +302,17 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(TrainArgs A) {
     for (int cc = 0; cc < kHid; cc += 16) {
       float dv[16];
       m.load16(cc, dv);
-      for (int i = 0; i < 16; ++i) {
-        const float a = load_bf16(sAct + l * kTileBytes, threadIdx.x, cc + i, kK);
-        dv[i] = a > 0.f ? dv[i] : 0.f;
-        sDf[threadIdx.x * kHid + cc + i] = dv[i];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 a8 = *reinterpret_cast<const uint4*>(sAct + l * kTileBytes + kmajor_offset(threadIdx.x, cc + 8 * h, kK));
+        const uint32_t w[4] = {a8.x, a8.y, a8.z, a8.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float a = __uint_as_float(i & 1 ? w[i / 2] & 0xffff0000u : w[i / 2] << 16);   // bf16 -> float
+          float& d = dv[8 * h + i];
+          d = a > 0.f ? d : 0.f;
+          sDf[threadIdx.x * kDfStride + cc + 8 * h + i] = d;
+        }
       }
       store8_bf16(sD, threadIdx.x, cc, kK, dv);
       store8_bf16(sD, threadIdx.x, cc + 8, kK, dv + 8);
@@ -451,9 +493,9 @@ int guide_train(Guide* g, cudaStream_t s, const float* recs, const int32_t* rec_
   const float b1 = 0.9f, b2 = 0.99f;
   cudaMemsetAsync(g->csum, 0, (size_t)steps * 4, s);
   cudaMemsetAsync(g->loss, 0, (size_t)steps * 4, s);
+  weight_sum_kernel<<<dim3(tiles, steps), kTile, 0, s>>>(recs, rec_count, cap, batch, seed, (uint64_t)g->t, g->csum);
   for (int k = 0; k < steps; ++k) {
     const uint64_t t = (uint64_t)g->t;
-    weight_sum_kernel<<<tiles, kTile, 0, s>>>(recs, rec_count, cap, batch, seed, t, g->csum + k);
     TrainArgs a{recs, rec_count, cap, batch, seed, t, alpha_fixed, g->csum + k, g->wf, g->wb, g->master, g->grad,
                 g->loss + k, g->err};
     guide_train_kernel<<<tiles, kTile, kTrainSmem, s>>>(a);

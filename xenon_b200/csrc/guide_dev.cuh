@@ -38,10 +38,6 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
   return r;
 }
 
-__device__ __forceinline__ float load_bf16(const uint8_t* tile, int r, int k, int K) {
-  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + xbd::kmajor_offset(r, k, K)));
-}
-
 // Row-major bf16 [rows][K] in global memory -> core-matrix tile in shared memory (block-wide).
 __device__ __forceinline__ void load_matrix(uint8_t* dst, const __nv_bfloat16* src, int rows, int K) {
   const int chunks = K / 8;
@@ -52,17 +48,22 @@ __device__ __forceinline__ void load_matrix(uint8_t* dst, const __nv_bfloat16* s
   }
 }
 
+// The biases b0 b1 b2 b3, contiguous, from the FP32 master vector (block-wide).
+__device__ __forceinline__ void load_biases(float* sBias, const float* master) {
+  for (int i = threadIdx.x; i < kBiasFloats; i += blockDim.x) {
+    const int l = i < 3 * kHid ? i / kHid : 3;
+    const int j = i < 3 * kHid ? i % kHid : i - 3 * kHid;
+    sBias[i] = master[off_b(l) + j];
+  }
+}
+
 // Forward weights (wf: 4 x [out][64] bf16) and biases (from the FP32 master vector) into shared
 // memory: W0 W1 W2 at kWBytes each, then W3; biases b0 b1 b2 b3 contiguous.
 __device__ __forceinline__ void load_forward_weights(uint8_t* sW, float* sBias, const __nv_bfloat16* wf,
                                                      const float* master) {
   for (int l = 0; l < 3; ++l) load_matrix(sW + l * kWBytes, wf + l * kHid * kK, kHid, kK);
   load_matrix(sW + 3 * kWBytes, wf + 3 * kHid * kK, kOut, kK);
-  for (int i = threadIdx.x; i < kBiasFloats; i += blockDim.x) {
-    const int l = i < 3 * kHid ? i / kHid : 3;
-    const int j = i < 3 * kHid ? i % kHid : i - 3 * kHid;
-    sBias[i] = master[off_b(l) + j];
-  }
+  load_biases(sBias, master);
 }
 
 // The 64 input features of one row into the A tile: sin/cos(2^k pi x) of the position in
