@@ -128,6 +128,8 @@ struct DevScene {
   int32_t sun_nee;   // XB_FLAG_SUN_NEE: directional lights weighted as delta lights (else the reference's 1e8)
   const float* sky_cdf;   // XB_FLAG_SKY_IS: kSkyBins + 1 cumulative bin masses over y in [-1, 1] (or nullptr)
   int32_t watertight;     // XB_FLAG_WATERTIGHT: ray_triangle_wt instead of Moller-Trumbore
+  float4 root_a, root_b;  // the TLAS root, as in nodes: for launches that are not captured, since a
+                          // refit changes it
   int32_t loose_boxes;    // some box holds a NaN, or a TLAS box is inverted: every ray is `odd` (SlabRay)
 };
 

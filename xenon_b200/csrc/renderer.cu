@@ -1189,6 +1189,7 @@ __global__ void resolve_kernel(const float4* accum, int W, int H, float inv_spp,
 // shared between calls (calls on different streams may overlap).
 // wide: rays and hits are 16-byte aligned (the ABI asks for 4), so records move as float4s.
 struct ApiIO {
+  static constexpr bool kCaptured = false;
   const xb_ray* rays;
   xb_hit* hits;
   unsigned long long* st;
@@ -1260,8 +1261,10 @@ struct ApiIO {
   __device__ __forceinline__ unsigned long long* stats() const { return st; }
 };
 
+// Blocks per SM: without the bounds the compiler takes 80 registers for any hits (1 M rays 564 ->
+// 626 us) or 92 for closest hits (4.19 M rays 335 -> 371 us).
 template <bool kAny>
-__global__ void __launch_bounds__(128) trace_api_persistent_kernel(DevScene sc, const xb_ray* rays, int n,
+__global__ void __launch_bounds__(128, kAny ? 7 : 6) trace_api_persistent_kernel(DevScene sc, const xb_ray* rays, int n,
                                                                    xb_hit* hits, unsigned long long* stats,
                                                                    int refill, bool wide) {
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1443,6 +1446,19 @@ int dev_upload(xb_renderer* r, const std::vector<T>& v, const T** out) {
   r->scene_mem.push_back(p);
   e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return set_err(r, XB_E_CUDA, "cudaMemcpy failed: %s", cudaGetErrorString(e));
+  *out = static_cast<const T*>(p);
+  return XB_OK;
+}
+
+// Device memory of the scene without contents.
+template <class T>
+int dev_array(xb_renderer* r, size_t n, const T** out) {
+  *out = nullptr;
+  if (n == 0) return XB_OK;
+  void* p = nullptr;
+  const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e != cudaSuccess) return set_err(r, XB_E_OOM, "cudaMalloc(%zu) failed: %s", n * sizeof(T), cudaGetErrorString(e));
+  r->scene_mem.push_back(p);
   *out = static_cast<const T*>(p);
   return XB_OK;
 }
@@ -2103,6 +2119,110 @@ __global__ void flip_rows_f64_kernel(const double* __restrict__ src, double* __r
   }
 }
 
+// ── scene upload: one mesh's arrays to the traversal's layout ────────────────────
+// (On the host this took 80 ms of a 1.31 M triangle scene's 125 ms from BVH build to first pick.)
+struct UploadStatus {
+  int32_t error, mesh;     // first error found, and where (see xb_upload_scene)
+  int32_t loose;           // a box with a NaN plane
+  uint32_t big_leaves;     // entries of DevScene::big_leaves in use
+};
+struct UploadArgs {
+  const float4* nodes;     // xb_bvh_node, two float4s each
+  const uint32_t* prims;
+  const int32_t* indices;
+  const int32_t* mat_ids;  // nullptr: 0
+  const float* v[3];
+  const float* n[3];       // nullptr: 0
+  size_t bytes;
+  int64_t node_base, slot_base;
+  int32_t vtx_base, num_nodes, num_tris, num_verts, num_materials, mesh;
+  uint32_t big_cap;
+  DevScene out;
+  UploadStatus* status;
+};
+
+__global__ void upload_mesh_kernel(UploadArgs a) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  auto fail = [&](int code) {
+    if (atomicCAS(&a.status->error, 0, code) == 0) a.status->mesh = a.mesh;
+  };
+  if (i < a.num_nodes) {
+    const float4 lo = a.nodes[2 * (size_t)i], hi = a.nodes[2 * (size_t)i + 1];   // mn, mx.x | mx.yz, child, count
+    uint32_t child = __float_as_uint(hi.z), entry = 0;
+    const uint32_t count = __float_as_uint(hi.w);
+    if (count > 0) {
+      if ((int64_t)child + count > a.num_tris) fail(1);
+      child += (uint32_t)a.slot_base;
+      entry = (count << 28) | child;
+      if (count >= kEntryEscape) {
+        const uint32_t k = atomicAdd(&a.status->big_leaves, 1u);
+        if (k < a.big_cap) const_cast<uint2*>(a.out.big_leaves)[k] = make_uint2(child, count);
+        entry = (kEntryEscape << 28) | k;
+      }
+    } else {
+      if ((int64_t)child + 1 >= a.num_nodes) fail(2);
+      entry = child + (uint32_t)a.node_base;
+    }
+    if (lo.x != lo.x || lo.y != lo.y || lo.z != lo.z || lo.w != lo.w || hi.x != hi.x || hi.y != hi.y) atomicExch(&a.status->loose, 1);
+    float4* q = const_cast<float4*>(a.out.nodes) + 2 * (size_t)(a.node_base + i);
+    q[0] = make_float4(lo.x, lo.y, lo.w, hi.x);
+    q[1] = make_float4(lo.z, hi.y, __uint_as_float(entry), hi.w);
+  }
+  if (i < a.num_tris) {
+    // triangle i of the mesh, and slot i's triangle
+    for (int k = 0; k < 3; ++k) {
+      const int32_t vi = a.indices[3 * (size_t)i + k];
+      if (vi < 0 || vi >= a.num_verts) fail(4);
+      const_cast<int32_t*>(a.out.tri_index)[3 * (size_t)(a.slot_base + i) + k] = a.vtx_base + vi;
+    }
+    const int32_t mat = a.mat_ids ? a.mat_ids[i] : 0;
+    if (mat < 0 || mat >= a.num_materials) fail(5);
+    const_cast<int32_t*>(a.out.tri_mat)[a.slot_base + i] = mat;
+    const uint32_t t = a.prims[i];
+    if (t >= (uint32_t)a.num_tris) {
+      fail(3);
+    } else {
+      for (int k = 0; k < 3; ++k) {
+        const int32_t vi = a.indices[3 * (size_t)t + k];
+        if (vi < 0 || vi >= a.num_verts) continue;   // reported where t is i
+        const_cast<float4*>(a.out.tris)[3 * (size_t)(a.slot_base + i) + k] =
+            make_float4(a.v[0][vi], a.v[1][vi], a.v[2][vi],
+                        __int_as_float(k == 0 ? (int)t : k == 1 ? (int)(a.slot_base + t) : 0));
+      }
+    }
+  }
+  if (i < a.num_verts) {
+    const_cast<float*>(a.out.nx)[a.vtx_base + i] = a.n[0] ? a.n[0][i] : 0.f;
+    const_cast<float*>(a.out.ny)[a.vtx_base + i] = a.n[1] ? a.n[1][i] : 0.f;
+    const_cast<float*>(a.out.nz)[a.vtx_base + i] = a.n[2] ? a.n[2][i] : 0.f;
+  }
+}
+
+// One mesh as the caller's arrays lie in the upload buffer, from `base` on.
+UploadArgs mesh_blob(const xb_mesh_view& mv, const xb_renderer::MeshLayout& ml, char* base, int num_materials) {
+  UploadArgs a{};
+  size_t at = 0;
+  auto take = [&](auto** p, bool there, size_t bytes) {
+    if (there) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + at);
+    at += there ? up256(bytes) : 0;
+  };
+  take(&a.nodes, true, 32 * (size_t)ml.num_nodes);
+  take(&a.prims, true, 4 * (size_t)ml.num_tris);
+  take(&a.indices, true, 12 * (size_t)ml.num_tris);
+  take(&a.mat_ids, mv.mat_ids != nullptr, 4 * (size_t)ml.num_tris);
+  for (int k = 0; k < 3; ++k) take(&a.v[k], true, 4 * (size_t)ml.num_verts);
+  for (int k = 0; k < 3; ++k) take(&a.n[k], mv.nx != nullptr, 4 * (size_t)ml.num_verts);
+  a.bytes = at;
+  a.node_base = ml.node_base;
+  a.slot_base = ml.slot_base;
+  a.vtx_base = ml.vtx_offset;
+  a.num_nodes = ml.num_nodes;
+  a.num_tris = ml.num_tris;
+  a.num_verts = ml.num_verts;
+  a.num_materials = num_materials;
+  return a;
+}
+
 // ── BLAS refit (xb_refit_mesh): one mesh's triangles and node boxes, topology kept ──────────
 // The passes are refit_kernels.h's, which the host refit (xb_scene_refit_mesh) runs as loops.
 __global__ void refit_finite_kernel(xb::RefitArgs a, const float* normals) {
@@ -2308,98 +2428,112 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   if (!v) return set_err(r, XB_E_INVALID, "xb_upload_scene: null view");
   CK(cudaStreamSynchronize(r->stream));
   free_scene(r);
-  // ── meshes: BLAS nodes (odd-aligned per mesh), slot-ordered triangles; the refit passes
-  // (refit_kernels.h, which states this layout) and the host refit's packing read it too ──
-  std::vector<float4> blas, tris;
-  std::vector<int32_t> tri_index, tri_mat, root_of(v->num_meshes, -1);
-  std::vector<float> nx, ny, nz;
+  // ── the meshes' places in the device arrays: BLAS nodes odd-aligned per mesh, slot-ordered
+  // triangles; the refit passes (refit_kernels.h, which states this layout) and the host refit's
+  // packing read it too. The TLAS nodes come first; a refit's has at most two per instance ──
+  const int64_t tlas_cap = std::max<int64_t>(v->num_tlas_nodes, 2 * (int64_t)v->num_instances);
+  std::vector<int32_t> root_of(v->num_meshes, -1);
   std::vector<DevMesh> meshes(v->num_meshes);
   r->mesh_layout.assign(v->num_meshes, xb_renderer::MeshLayout());
-  int64_t slot_base = 0, tri_base = 0, vtx_base = 0;
-  // the TLAS nodes' places at the front; a refit's TLAS has at most two nodes per instance
-  const int64_t tlas_cap = std::max<int64_t>(v->num_tlas_nodes, 2 * (int64_t)v->num_instances);
-  blas.resize(2 * (size_t)tlas_cap, make_float4(0, 0, 0, 0));
-  bool loose = false;
-  std::vector<uint2> big_leaves;
-  size_t nn = 0, nt = 0, nv = 0;
-  for (int m = 0; m < v->num_meshes; ++m) {
-    nn += std::max(v->meshes[m].num_blas_nodes, 0) + 2;
-    nt += std::max(v->meshes[m].num_triangles, 0);
-    nv += std::max(v->meshes[m].num_vertices, 0);
-  }
-  blas.reserve(blas.size() + 2 * nn);
-  tris.reserve(3 * nt);
-  tri_index.reserve(3 * nt);
-  tri_mat.reserve(nt);
-  for (auto* c : {&nx, &ny, &nz}) c->reserve(nv);
+  int64_t node_count = tlas_cap, slot_base = 0, vtx_base = 0;
+  size_t blob = 0;
   for (int m = 0; m < v->num_meshes; ++m) {
     const xb_mesh_view& mv = v->meshes[m];
     if (mv.num_triangles > 0 && (!mv.blas_nodes || mv.num_blas_nodes <= 0 || !mv.blas_prims))
       return set_err(r, XB_E_INVALID, "mesh %d has no BLAS", m);
-    if ((blas.size() / 2) % 2 == 0) { blas.push_back(make_float4(0, 0, 0, 0)); blas.push_back(make_float4(0, 0, 0, 0)); }
-    const int64_t node_base = (int64_t)blas.size() / 2;
-    if (mv.num_blas_nodes > 0) root_of[m] = (int32_t)node_base;
+    node_count += (node_count + 1) & 1;
     xb_renderer::MeshLayout& ml = r->mesh_layout[m];
-    ml.node_base = node_base;
+    ml.node_base = node_count;
     ml.slot_base = slot_base;
     ml.num_nodes = mv.num_blas_nodes > 0 ? mv.num_blas_nodes : 0;
-    ml.num_tris = mv.num_triangles;
-    ml.num_verts = mv.num_vertices;
-    ml.tri_offset = (int32_t)tri_base;
-    ml.vtx_offset = (int32_t)vtx_base;
-    ml.has_normals = mv.nx != nullptr;
-    if (ml.num_nodes > 0) ml.root = mv.blas_nodes[0];
-    for (int i = 0; i < mv.num_blas_nodes; ++i) {
-      const xb_bvh_node& nd = mv.blas_nodes[i];
-      uint32_t child;
-      if (nd.count > 0) {
-        if ((int64_t)nd.child + nd.count > mv.num_triangles) return set_err(r, XB_E_INVALID, "mesh %d BLAS leaf out of range", m);
-        child = (uint32_t)(slot_base + nd.child);
-      } else {
-        if ((int64_t)nd.child + 1 >= mv.num_blas_nodes) return set_err(r, XB_E_INVALID, "mesh %d BLAS child out of range", m);
-        child = (uint32_t)(node_base + nd.child);
-      }
-      blas.push_back(make_float4(nd.mn[0], nd.mn[1], nd.mx[0], nd.mx[1]));
-      uint32_t entry = (nd.count << 28) | child;
-      if (nd.count >= kEntryEscape) {
-        entry = (kEntryEscape << 28) | (uint32_t)big_leaves.size();
-        big_leaves.push_back(make_uint2(child, nd.count));
-      }
-      blas.push_back(make_float4(nd.mn[2], nd.mx[2], u32_bits_to_f(entry), u32_bits_to_f(nd.count)));
-      for (int k = 0; k < 3; ++k) loose = loose || nd.mn[k] != nd.mn[k] || nd.mx[k] != nd.mx[k];
+    ml.num_tris = std::max(mv.num_triangles, 0);
+    ml.num_verts = std::max(mv.num_vertices, 0);
+    ml.tri_offset = meshes[m].tri_offset = (int32_t)slot_base;
+    ml.vtx_offset = meshes[m].vtx_offset = (int32_t)vtx_base;
+    ml.has_normals = meshes[m].has_normals = mv.nx != nullptr;
+    if (ml.num_nodes > 0) {
+      ml.root = mv.blas_nodes[0];
+      root_of[m] = (int32_t)ml.node_base;
     }
-    for (int s = 0; s < mv.num_triangles; ++s) {
-      const uint32_t t = mv.blas_prims[s];
-      if ((int)t >= mv.num_triangles) return set_err(r, XB_E_INVALID, "mesh %d prim index out of range", m);
-      const int i0 = mv.indices[3 * t], i1 = mv.indices[3 * t + 1], i2 = mv.indices[3 * t + 2];
-      tris.push_back(make_float4(mv.vx[i0], mv.vy[i0], mv.vz[i0], i32_bits_to_f((int)t)));
-      tris.push_back(make_float4(mv.vx[i1], mv.vy[i1], mv.vz[i1], i32_bits_to_f((int)(tri_base + t))));
-      tris.push_back(make_float4(mv.vx[i2], mv.vy[i2], mv.vz[i2], 0.f));
-    }
-    for (int t = 0; t < mv.num_triangles; ++t) {
-      for (int k = 0; k < 3; ++k) {
-        const int vi = mv.indices[3 * t + k];
-        if (vi < 0 || vi >= mv.num_vertices) return set_err(r, XB_E_INVALID, "mesh %d vertex index out of range", m);
-        tri_index.push_back((int32_t)(vtx_base + vi));
-      }
-      const int mid = mv.mat_ids ? mv.mat_ids[t] : 0;
-      if (mid < 0 || mid >= v->num_materials) return set_err(r, XB_E_INVALID, "mesh %d triangle %d material %d out of range", m, t, mid);
-      tri_mat.push_back(mid);
-    }
-    meshes[m].tri_offset = (int32_t)tri_base;
-    meshes[m].vtx_offset = (int32_t)vtx_base;
-    meshes[m].has_normals = mv.nx != nullptr;
-    for (int i = 0; i < mv.num_vertices; ++i) {
-      nx.push_back(mv.nx ? mv.nx[i] : 0.f);
-      ny.push_back(mv.ny ? mv.ny[i] : 0.f);
-      nz.push_back(mv.nz ? mv.nz[i] : 0.f);
-    }
-    slot_base += mv.num_triangles;
-    tri_base += mv.num_triangles;
-    vtx_base += mv.num_vertices;
+    node_count += ml.num_nodes;
+    slot_base += ml.num_tris;
+    vtx_base += ml.num_verts;
+    blob = std::max(blob, mesh_blob(mv, ml, nullptr, 0).bytes);
   }
-  if (blas.size() / 2 >= (1u << 28) || slot_base >= (1 << 28))
+  if (node_count >= (1u << 28) || slot_base >= (1 << 28))
     return set_err(r, XB_E_UNSUPPORTED, "scene too large: more than 2^28 BLAS nodes or triangles");
+  std::vector<uint2> big_leaves;
+  std::vector<float4> tlas;
+  bool loose_tlas = false;
+  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves, loose_tlas))
+    return set_err(r, XB_E_INVALID, "a TLAS node has two parents, or the TLAS is too large");
+  DevScene& sc = r->scene;
+  std::memset(&sc, 0, sizeof(sc));
+  if ((rc = dev_array(r, 2 * (size_t)node_count, &sc.nodes))) return rc;
+  if ((rc = dev_array(r, 3 * (size_t)slot_base, &sc.tris))) return rc;
+  if ((rc = dev_array(r, 3 * (size_t)slot_base, &sc.tri_index))) return rc;
+  if ((rc = dev_array(r, (size_t)slot_base, &sc.tri_mat))) return rc;
+  if ((rc = dev_array(r, (size_t)vtx_base, &sc.nx))) return rc;
+  if ((rc = dev_array(r, (size_t)vtx_base, &sc.ny))) return rc;
+  if ((rc = dev_array(r, (size_t)vtx_base, &sc.nz))) return rc;
+  if (!tlas.empty())
+    CK(cudaMemcpyAsync(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice, r->stream));
+  UploadStatus up{};
+  {
+    const Scratch mem(r, up256(blob) + sizeof(UploadStatus));
+    if (!mem.p) return set_err(r, XB_E_OOM, "xb_upload_scene: out of device memory");
+    UploadStatus* const status = reinterpret_cast<UploadStatus*>(static_cast<char*>(mem.p) + up256(blob));
+    // leaves that an entry cannot hold are 15 triangles or more; should leaves overlap so that there
+    // are more, the second turn has room for all
+    const uint32_t first = (uint32_t)big_leaves.size();
+    uint32_t cap = first + (uint32_t)(slot_base / kEntryEscape) + 1;
+    for (int turn = 0; turn < 2; ++turn) {
+      if ((rc = dev_array(r, cap, &sc.big_leaves))) return rc;
+      up = UploadStatus{};
+      up.big_leaves = first;
+      CK(cudaMemcpyAsync(status, &up, sizeof(up), cudaMemcpyHostToDevice, r->stream));
+      std::vector<char> host;
+      for (int m = 0; m < v->num_meshes; ++m) {
+        const xb_renderer::MeshLayout& ml = r->mesh_layout[m];
+        const xb_mesh_view& mv = v->meshes[m];
+        const int n = std::max(std::max(ml.num_nodes, ml.num_tris), ml.num_verts);
+        if (n == 0) continue;
+        UploadArgs a = mesh_blob(mv, ml, static_cast<char*>(mem.p), v->num_materials);
+        // a small mesh's arrays go up as one copy, a large one's each from where they are
+        const bool together = a.bytes <= (size_t)256 << 10;
+        if (together) host.assign(a.bytes, 0);
+        const struct { const void* src; const void* dst; size_t bytes; } parts[] = {
+            {mv.blas_nodes, a.nodes, 32 * (size_t)ml.num_nodes}, {mv.blas_prims, a.prims, 4 * (size_t)ml.num_tris},
+            {mv.indices, a.indices, 12 * (size_t)ml.num_tris}, {mv.mat_ids, a.mat_ids, 4 * (size_t)ml.num_tris},
+            {mv.vx, a.v[0], 4 * (size_t)ml.num_verts}, {mv.vy, a.v[1], 4 * (size_t)ml.num_verts},
+            {mv.vz, a.v[2], 4 * (size_t)ml.num_verts}, {mv.nx, a.n[0], 4 * (size_t)ml.num_verts},
+            {mv.nx ? mv.ny : nullptr, a.n[1], 4 * (size_t)ml.num_verts}, {mv.nx ? mv.nz : nullptr, a.n[2], 4 * (size_t)ml.num_verts}};
+        for (const auto& q : parts) {
+          if (!q.src || !q.bytes) continue;
+          if (together) std::memcpy(host.data() + (static_cast<const char*>(q.dst) - static_cast<char*>(mem.p)), q.src, q.bytes);
+          else CK(cudaMemcpyAsync(const_cast<void*>(q.dst), q.src, q.bytes, cudaMemcpyHostToDevice, r->stream));
+        }
+        if (together) CK(cudaMemcpyAsync(mem.p, host.data(), a.bytes, cudaMemcpyHostToDevice, r->stream));
+        a.mesh = m;
+        a.big_cap = cap;
+        a.out = sc;
+        a.status = status;
+        upload_mesh_kernel<<<(n + 255) / 256, 256, 0, r->stream>>>(a);
+      }
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(&up, status, sizeof(up), cudaMemcpyDeviceToHost, r->stream));
+      CK(cudaStreamSynchronize(r->stream));
+      if (up.error) {
+        static const char* const what[] = {"", "BLAS leaf out of range", "BLAS child out of range", "prim index out of range",
+                                           "vertex index out of range", "triangle material out of range"};
+        return set_err(r, XB_E_INVALID, "mesh %d %s", up.mesh, what[up.error]);
+      }
+      if (up.big_leaves <= cap) break;
+      cap = up.big_leaves;
+    }
+    if (first > 0)
+      CK(cudaMemcpy(const_cast<uint2*>(sc.big_leaves), big_leaves.data(), first * sizeof(uint2), cudaMemcpyHostToDevice));
+  }
   // ── analytic prims in PrimBLAS slot order ──
   std::vector<float4> pnodes, prims;
   for (int i = 0; i < v->num_prim_nodes; ++i) {
@@ -2418,11 +2552,6 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
     prims.push_back(make_float4(q.p[8], q.p[9], 0.f, 0.f));
   }
   // ── TLAS and instances ──
-  std::vector<float4> tlas;
-  bool loose_tlas = false;
-  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves, loose_tlas))
-    return set_err(r, XB_E_INVALID, "a TLAS node has two parents, or the TLAS is too large");
-  std::copy(tlas.begin(), tlas.end(), blas.begin());
   std::vector<DevInstance> insts(v->num_instances);
   r->inst_geom.assign(v->num_instances, 0);
   r->inst_l2w.assign(v->num_instances, xb::Affine());
@@ -2443,7 +2572,12 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
       if (iv.geom < 0 || iv.geom >= v->num_meshes) return set_err(r, XB_E_INVALID, "instance %d: bad mesh %d", i, iv.geom);
       if (root_of[iv.geom] < 0) return set_err(r, XB_E_INVALID, "instance %d uses an empty mesh", i);
       d.kind = 0; d.mesh = iv.geom;
-      std::memcpy(&d.root, &blas[2 * (size_t)root_of[iv.geom] + 1].z, sizeof(d.root));
+      const xb_bvh_node& root = r->mesh_layout[iv.geom].root;
+      if (root.count < kEntryEscape)
+        d.root = (root.count << 28) | (uint32_t)(root.child + (root.count ? r->mesh_layout[iv.geom].slot_base : root_of[iv.geom]));
+      else
+        CK(cudaMemcpy(&d.root, reinterpret_cast<const char*>(sc.nodes + 2 * (size_t)root_of[iv.geom] + 1) + 8, 4,
+                      cudaMemcpyDeviceToHost));
     }
   }
   r->inst_dev = insts;
@@ -2479,20 +2613,10 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
     xb::sun_emission(v->suns[i], s.emission);
     suns.push_back(s);
   }
-  DevScene& sc = r->scene;
-  std::memset(&sc, 0, sizeof(sc));
-  if ((rc = dev_upload(r, blas, &sc.nodes))) return rc;
-  if ((rc = dev_upload(r, tris, &sc.tris))) return rc;
-  if ((rc = dev_upload(r, big_leaves, &sc.big_leaves))) return rc;
   if ((rc = dev_upload(r, pnodes, &sc.pnodes))) return rc;
   if ((rc = dev_upload(r, prims, &sc.prims))) return rc;
   if ((rc = dev_upload(r, ordered, &sc.inst))) return rc;
   if ((rc = dev_upload(r, meshes, &sc.meshes))) return rc;
-  if ((rc = dev_upload(r, tri_index, &sc.tri_index))) return rc;
-  if ((rc = dev_upload(r, tri_mat, &sc.tri_mat))) return rc;
-  if ((rc = dev_upload(r, nx, &sc.nx))) return rc;
-  if ((rc = dev_upload(r, ny, &sc.ny))) return rc;
-  if ((rc = dev_upload(r, nz, &sc.nz))) return rc;
   if ((rc = dev_upload(r, mats, &sc.mats))) return rc;
   if ((rc = dev_upload(r, lights, &sc.lights))) return rc;
   if ((rc = dev_upload(r, suns, &sc.suns))) return rc;
@@ -2505,9 +2629,10 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.num_lights = v->num_lights;
   sc.num_suns = v->num_suns;
   sc.num_tlas_nodes = v->num_tlas_nodes;
+  if (!tlas.empty()) { sc.root_a = tlas[0]; sc.root_b = tlas[1]; }
   r->tlas_cap = tlas_cap;
-  r->big_leaves = (int64_t)big_leaves.size();
-  r->loose_blas = loose;
+  r->big_leaves = up.big_leaves;
+  r->loose_blas = up.loose != 0;
   sc.num_materials = v->num_materials;
   std::memcpy(sc.sky_zenith, v->sky.zenith, sizeof(sc.sky_zenith));
   std::memcpy(sc.sky_horizon, v->sky.horizon, sizeof(sc.sky_horizon));
@@ -2515,7 +2640,7 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.sky_inv_sharpness = 1.0f / v->sky.sharpness;
   sc.sky_intensity = v->sky.intensity;
   sc.sun_nee = (r->cfg.flags & XB_FLAG_SUN_NEE) != 0;
-  sc.loose_boxes = loose || loose_tlas;
+  sc.loose_boxes = up.loose != 0 || loose_tlas;
   sc.watertight = (r->cfg.flags & XB_FLAG_WATERTIGHT) != 0;
   if ((r->cfg.flags & XB_FLAG_SKY_IS) && sc.sky_intensity > 0.f) {
     std::vector<float> cdf;
@@ -2653,7 +2778,9 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
       r->scene_hi[k] = nodes[0].mx[k];
     }
   }
-  // the captured bounce loops hold the scene's pointers and counts, and guided ones its bounds
+  // the captured bounce loops hold the scene's pointers and counts (the root they read from its
+  // array), and guided ones its bounds
+  if (!tlas.empty()) { before.root_a = sc.root_a = tlas[0]; before.root_b = sc.root_b = tlas[1]; }
   if (std::memcmp(&before, &sc, sizeof(sc)) != 0 || (r->guide && moved)) drop_graphs(r);
   return XB_OK;
 }

@@ -54,6 +54,7 @@ struct TraceQueue {
 
 // Where a warp's rays come from and where their answers go: the renderer's queues, the rays
 // taken from a shared cursor (a TraceQueue; xb_trace_rays_device has its own, in renderer.cu).
+//   kCaptured               the launch may be part of a captured graph
 //   end()                   one past the last ray index this warp may take
 //   lanes()                 how many of the warp's lanes take rays
 //   grab(lane, leader, k)   the first of k consecutive ray indices for the warp's idle lanes
@@ -69,6 +70,7 @@ struct TraceQueue {
 // same way was 4-15 % slower. A warp's first rays are its own by its number; only later ones come
 // from the cursor.
 struct QueueIO {
+  static constexpr bool kCaptured = true;
   TraceQueue q;
   int n, per_warp;
   bool first;
@@ -269,8 +271,8 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, IO& io, int
           occluded = false;
           if (sc.num_tlas_nodes > 0) {
             if (kCount) cnt.tlas++;
-            float4 root_a, root_b;
-            ldg8(sc.nodes, root_a, root_b);
+            float4 root_a = sc.root_a, root_b = sc.root_b;
+            if constexpr (IO::kCaptured) ldg8(sc.nodes, root_a, root_b);
             float tn;
             if (odd ? aabb_fast(root_a, root_b, winv, wo, wd, tmin, t_best, tn)
                     : sr.slab(root_a, root_b, tmin, t_best, tn)) {
