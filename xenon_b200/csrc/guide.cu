@@ -27,6 +27,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/xenon_b200.h"
@@ -385,6 +386,7 @@ __global__ void finalize_records_kernel(float* recs, const int32_t* rec_count, i
 }  // namespace
 
 struct Guide {
+  void* mem = nullptr;         // one allocation of everything below but the records
   float* master = nullptr;     // kParams FP32
   float* grad = nullptr;
   float* mom = nullptr;
@@ -406,12 +408,23 @@ int guide_create(Guide** out, uint64_t seed, int rec_cap) {
   if (!g) return XB_E_OOM;
   g->max_steps = kMaxTrainSteps;
   g->rec_cap = std::max(0, rec_cap);
-  bool ok = cudaMalloc(&g->master, kParams * 4) == cudaSuccess && cudaMalloc(&g->grad, kParams * 4) == cudaSuccess &&
-            cudaMalloc(&g->mom, kParams * 4) == cudaSuccess && cudaMalloc(&g->vel, kParams * 4) == cudaSuccess &&
-            cudaMalloc(&g->wf, 4 * kHid * kK * 2) == cudaSuccess && cudaMalloc(&g->wb, 4 * kHid * kK * 2) == cudaSuccess &&
-            cudaMalloc(&g->csum, g->max_steps * 4) == cudaSuccess &&
-            cudaMalloc(&g->loss, g->max_steps * 4) == cudaSuccess && cudaMalloc(&g->err, 4) == cudaSuccess &&
-            cudaMalloc(&g->rec_count, 4) == cudaSuccess;
+  // one allocation, cleared in one go (eleven before: a network is made for each xb_guide_* call)
+  size_t at = 0;
+  auto place = [&](auto** p, size_t bytes) {
+    *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(static_cast<char*>(g->mem) + at);
+    at += (bytes + 255) & ~(size_t)255;
+  };
+  auto layout = [&]() {
+    at = 0;
+    for (float** p : {&g->master, &g->grad, &g->mom, &g->vel}) place(p, kParams * 4);
+    for (__nv_bfloat16** p : {&g->wf, &g->wb}) place(p, 4 * kHid * kK * 2);
+    for (float** p : {&g->csum, &g->loss}) place(p, (size_t)g->max_steps * 4);
+    place(&g->err, 4);
+    place(&g->rec_count, 4);
+  };
+  layout();
+  bool ok = cudaMalloc(&g->mem, at) == cudaSuccess;
+  layout();
   if (ok && g->rec_cap > 0) ok = cudaMalloc(&g->recs, (size_t)g->rec_cap * kRecFloats * 4) == cudaSuccess;
   if (!ok) { guide_destroy(g); return XB_E_OOM; }
   // He-uniform hidden layers and a 0.1-scaled output layer (as the oracle's init_params), drawn
@@ -431,14 +444,8 @@ int guide_create(Guide** out, uint64_t seed, int rec_cap) {
     const double bound = std::sqrt(6.0 / kK) * (l == 3 ? 0.1 : 1.0);
     for (int i = 0; i < outs * kK; ++i) p[off_w(l) + i] = (float)((2.0 * next() - 1.0) * bound);
   }
-  bool cok = cudaMemcpy(g->master, p.data(), kParams * 4, cudaMemcpyHostToDevice) == cudaSuccess;
-  cok &= cudaMemset(g->grad, 0, kParams * 4) == cudaSuccess;
-  cok &= cudaMemset(g->mom, 0, kParams * 4) == cudaSuccess;
-  cok &= cudaMemset(g->vel, 0, kParams * 4) == cudaSuccess;
-  cok &= cudaMemset(g->wf, 0, 4 * kHid * kK * 2) == cudaSuccess;
-  cok &= cudaMemset(g->wb, 0, 4 * kHid * kK * 2) == cudaSuccess;
-  cok &= cudaMemset(g->err, 0, 4) == cudaSuccess;
-  cok &= cudaMemset(g->rec_count, 0, 4) == cudaSuccess;
+  bool cok = cudaMemset(g->mem, 0, at) == cudaSuccess;
+  cok &= cudaMemcpy(g->master, p.data(), kParams * 4, cudaMemcpyHostToDevice) == cudaSuccess;
   cok &= cudaFuncSetAttribute(guide_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem) == cudaSuccess;
   cok &= cudaFuncSetAttribute(guide_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem) == cudaSuccess;
   guide_sync_bf16(g, 0);
@@ -449,9 +456,7 @@ int guide_create(Guide** out, uint64_t seed, int rec_cap) {
 
 void guide_destroy(Guide* g) {
   if (!g) return;
-  void* ptrs[] = {g->master, g->grad, g->mom, g->vel, g->wf, g->wb, g->csum, g->loss, g->err,
-                  g->recs, g->rec_count};
-  for (void* q : ptrs) if (q) cudaFree(q);
+  for (void* q : {g->mem, (void*)g->recs}) if (q) cudaFree(q);
   delete g;
 }
 
