@@ -950,7 +950,7 @@ def main():
         r.set_tuning(waves=lanes)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-                "peak_source": peaks["source"], "kernel": "extend_kernel (closest-hit traversal)",
+                "peak_source": peaks["source"], "kernel": "extend_persistent_kernel (closest-hit traversal)",
                 "algorithmic_bytes_per_ray": ext_bytes_per_ray,
                 "algorithmic_bytes_per_launch": ext_bytes / max(prof.extend_launches, 1),
                 "extend_busy_ms_per_step": ext_busy_ms / n_prof,
