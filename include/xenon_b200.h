@@ -320,7 +320,8 @@ int  xb_upload_scene(xb_renderer *r, const xb_scene_view *view);
  * emitter geometry is built on the host at upload; refit the host scene and upload again).
  * Synchronises the render stream. The
  * arrays are rewritten in place, so ray queries issued on caller streams (xb_trace_rays_device,
- * xb_trace_rays_noalloc) must have finished before this call. If the uploaded BLAS turns out to
+ * xb_trace_rays_noalloc) must have finished before this call; ones captured into a CUDA graph may be
+ * replayed after it and trace the refitted scene (not after an upload). If the uploaded BLAS turns out to
  * be malformed (XB_E_INVALID), some of it has already been rewritten: the renderer then holds no
  * scene (later calls fail with XB_E_STATE) until the scene is uploaded again. The accumulated
  * image is kept: call xb_reset for frames of a moving scene. No reference counterpart: the

@@ -8,7 +8,8 @@
 //             (src/geometry/blas.cpp:103-152). entry is the node as the traversal stacks it (see
 //             kLeafEntry). The order of the six planes makes each register pair of the load an
 //             operand of the packed (f32x2) slab arithmetic. key: a BLAS node's triangle count
-//             (the refit reads it), a TLAS node's centre on its parent's widest axis.
+//             (the refit reads it), a TLAS node's centre on its parent's widest axis, in the
+//             root 1 when a TLAS box holds a NaN or is inverted (else 0).
 //   tris      float4[3 * S]: the triangle of BLAS prim slot s, pre-gathered in slot order
 //             {v0, local tri id}, {v1, global tri id}, {v2, -}: a leaf's triangles are
 //             contiguous 48 B records (src/geometry/mesh.h:37-44 gather, done once on upload).
@@ -128,9 +129,8 @@ struct DevScene {
   int32_t sun_nee;   // XB_FLAG_SUN_NEE: directional lights weighted as delta lights (else the reference's 1e8)
   const float* sky_cdf;   // XB_FLAG_SKY_IS: kSkyBins + 1 cumulative bin masses over y in [-1, 1] (or nullptr)
   int32_t watertight;     // XB_FLAG_WATERTIGHT: ray_triangle_wt instead of Moller-Trumbore
-  float4 root_a, root_b;  // the TLAS root, as in nodes: for launches that are not captured, since a
-                          // refit changes it
-  int32_t loose_boxes;    // some box holds a NaN, or a TLAS box is inverted: every ray is `odd` (SlabRay)
+  int32_t loose_boxes;    // some BLAS box holds a NaN: every ray is `odd` (SlabRay). The TLAS's own such
+                          // flag is in its root (see nodes): a refit rewrites that
 };
 
 // The sky's luminance distribution over directions. The gradient sky (Environment::evaluate)

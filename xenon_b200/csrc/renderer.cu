@@ -202,7 +202,6 @@ struct xb_renderer {
   bool has_prim_root = false;
   int64_t tlas_cap = 0;         // TLAS nodes that fit at the front of the device's node array
   int64_t big_leaves = 0;       // entries of its big_leaves
-  bool loose_blas = false;      // see DevScene::loose_boxes
   void* refit_mem = nullptr;
   size_t refit_bytes = 0;
 };
@@ -1189,7 +1188,6 @@ __global__ void resolve_kernel(const float4* accum, int W, int H, float inv_spp,
 // shared between calls (calls on different streams may overlap).
 // wide: rays and hits are 16-byte aligned (the ABI asks for 4), so records move as float4s.
 struct ApiIO {
-  static constexpr bool kCaptured = false;
   const xb_ray* rays;
   xb_hit* hits;
   unsigned long long* st;
@@ -1473,8 +1471,9 @@ float4 node_hi(const xb_bvh_node& n, uint32_t child) {
 // exist. False when a node has two parents (its pair's key would serve one of them) or is the
 // root's parent, or there are too many.
 bool pack_tlas(const xb_bvh_node* nodes, int32_t n, int32_t num_inst, std::vector<float4>& out,
-               std::vector<uint2>& big_leaves, bool& loose) {
+               std::vector<uint2>& big_leaves) {
   if (n >= (1 << 27)) return false;
+  bool loose = false;
   std::vector<uint32_t> entry(n);
   std::vector<float> key(n, 0.f);
   std::vector<uint8_t> seen(n, 0);
@@ -1502,6 +1501,7 @@ bool pack_tlas(const xb_bvh_node* nodes, int32_t n, int32_t num_inst, std::vecto
       entry[ch] |= c == 0 ? (ax & 1u) : (ax >> 1);
     }
   }
+  if (loose) key[0] = 1.f;
   out.clear();
   for (int32_t i = 0; i < n; ++i) {
     const xb_bvh_node& nd = nodes[i];
@@ -2464,8 +2464,7 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
     return set_err(r, XB_E_UNSUPPORTED, "scene too large: more than 2^28 BLAS nodes or triangles");
   std::vector<uint2> big_leaves;
   std::vector<float4> tlas;
-  bool loose_tlas = false;
-  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves, loose_tlas))
+  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves))
     return set_err(r, XB_E_INVALID, "a TLAS node has two parents, or the TLAS is too large");
   DevScene& sc = r->scene;
   std::memset(&sc, 0, sizeof(sc));
@@ -2629,10 +2628,8 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.num_lights = v->num_lights;
   sc.num_suns = v->num_suns;
   sc.num_tlas_nodes = v->num_tlas_nodes;
-  if (!tlas.empty()) { sc.root_a = tlas[0]; sc.root_b = tlas[1]; }
   r->tlas_cap = tlas_cap;
   r->big_leaves = up.big_leaves;
-  r->loose_blas = up.loose != 0;
   sc.num_materials = v->num_materials;
   std::memcpy(sc.sky_zenith, v->sky.zenith, sizeof(sc.sky_zenith));
   std::memcpy(sc.sky_horizon, v->sky.horizon, sizeof(sc.sky_horizon));
@@ -2640,7 +2637,7 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.sky_inv_sharpness = 1.0f / v->sky.sharpness;
   sc.sky_intensity = v->sky.intensity;
   sc.sun_nee = (r->cfg.flags & XB_FLAG_SUN_NEE) != 0;
-  sc.loose_boxes = up.loose != 0 || loose_tlas;
+  sc.loose_boxes = up.loose != 0;
   sc.watertight = (r->cfg.flags & XB_FLAG_WATERTIGHT) != 0;
   if ((r->cfg.flags & XB_FLAG_SKY_IS) && sc.sky_intensity > 0.f) {
     std::vector<float> cdf;
@@ -2754,16 +2751,14 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   }
   std::vector<float4> tlas;
   std::vector<uint2> big((size_t)r->big_leaves);
-  bool loose_tlas = false;
   DevScene& sc = r->scene;
   // every leaf of this TLAS is one instance, so it fits the array and adds no big leaf
-  if (!pack_tlas(nodes.data(), (int)nodes.size(), (int)r->inst_geom.size(), tlas, big, loose_tlas) ||
+  if (!pack_tlas(nodes.data(), (int)nodes.size(), (int)r->inst_geom.size(), tlas, big) ||
       (int64_t)nodes.size() > r->tlas_cap || (int64_t)big.size() > r->big_leaves)
     return set_err(r, XB_E_UNSUPPORTED, "xb_refit_mesh: the rebuilt TLAS does not fit the uploaded scene's");
   if (!tlas.empty()) {
     CK(cudaMemcpy(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice));
   }
-  sc.loose_boxes = r->loose_blas || loose_tlas;
   if (!order.empty()) {
     const std::vector<DevInstance> ordered = in_tlas_order(r->inst_dev, order.data(), order.size());
     CK(cudaMemcpy(const_cast<DevInstance*>(sc.inst), ordered.data(), ordered.size() * sizeof(DevInstance),
@@ -2778,9 +2773,7 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
       r->scene_hi[k] = nodes[0].mx[k];
     }
   }
-  // the captured bounce loops hold the scene's pointers and counts (the root they read from its
-  // array), and guided ones its bounds
-  if (!tlas.empty()) { before.root_a = sc.root_a = tlas[0]; before.root_b = sc.root_b = tlas[1]; }
+  // the captured bounce loops hold the scene's pointers and counts, and guided ones its bounds
   if (std::memcmp(&before, &sc, sizeof(sc)) != 0 || (r->guide && moved)) drop_graphs(r);
   return XB_OK;
 }

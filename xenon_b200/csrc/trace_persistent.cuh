@@ -54,7 +54,6 @@ struct TraceQueue {
 
 // Where a warp's rays come from and where their answers go: the renderer's queues, the rays
 // taken from a shared cursor (a TraceQueue; xb_trace_rays_device has its own, in renderer.cu).
-//   kCaptured               the launch may be part of a captured graph
 //   end()                   one past the last ray index this warp may take
 //   lanes()                 how many of the warp's lanes take rays
 //   grab(lane, leader, k)   the first of k consecutive ray indices for the warp's idle lanes
@@ -70,7 +69,6 @@ struct TraceQueue {
 // same way was 4-15 % slower. A warp's first rays are its own by its number; only later ones come
 // from the cursor.
 struct QueueIO {
-  static constexpr bool kCaptured = true;
   TraceQueue q;
   int n, per_warp;
   bool first;
@@ -149,6 +147,12 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, IO& io, int
     w[W_U * kShStride] = u; w[W_V * kShStride] = v;
     w[W_PRIM * kShStride] = __int_as_float(prim); w[W_INST * kShStride] = __int_as_float(inst);
   };
+  // The TLAS root, read by the launch (which may be part of a captured graph) from where a refit
+  // moves it; a copy per warp, for new rays.
+  __shared__ float4 s_root[2 * (kShStride / 32)];
+  const int warp = threadIdx.x >> 5;
+  if (lane < 2 && sc.num_tlas_nodes > 0) s_root[2 * warp + lane] = ldg4(sc.nodes + lane);
+  __syncwarp();
   TraversalCounters cnt{0, 0, 0, 0};
   bool overflow = false;
 
@@ -271,8 +275,8 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, IO& io, int
           occluded = false;
           if (sc.num_tlas_nodes > 0) {
             if (kCount) cnt.tlas++;
-            float4 root_a = sc.root_a, root_b = sc.root_b;
-            if constexpr (IO::kCaptured) ldg8(sc.nodes, root_a, root_b);
+            const float4 root_a = s_root[2 * warp], root_b = s_root[2 * warp + 1];
+            odd = world_odd = world_odd || root_b.w != 0.f;
             float tn;
             if (odd ? aabb_fast(root_a, root_b, winv, wo, wd, tmin, t_best, tn)
                     : sr.slab(root_a, root_b, tmin, t_best, tn)) {
