@@ -1434,6 +1434,7 @@ void free_wave(xb_renderer* r) {
   r->lanes_alloc = 0;
 }
 
+// v in device memory of its own, once r->stream has been waited for (v lives until then).
 template <class T>
 int dev_upload(xb_renderer* r, const std::vector<T>& v, const T** out) {
   *out = nullptr;
@@ -1442,8 +1443,8 @@ int dev_upload(xb_renderer* r, const std::vector<T>& v, const T** out) {
   cudaError_t e = cudaMalloc(&p, v.size() * sizeof(T));
   if (e != cudaSuccess) return set_err(r, XB_E_OOM, "cudaMalloc(%zu) failed: %s", v.size() * sizeof(T), cudaGetErrorString(e));
   r->scene_mem.push_back(p);
-  e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return set_err(r, XB_E_CUDA, "cudaMemcpy failed: %s", cudaGetErrorString(e));
+  e = cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, r->stream);
+  if (e != cudaSuccess) return set_err(r, XB_E_CUDA, "cudaMemcpyAsync failed: %s", cudaGetErrorString(e));
   *out = static_cast<const T*>(p);
   return XB_OK;
 }
@@ -2359,8 +2360,8 @@ int xb_create(const xb_config* cfg, xb_renderer** out) {
   }
   rc = xb_reset(r);
   if (rc != XB_OK) return bail(rc);
-  if (cudaMemset(r->stats, 0, STAT_COUNT * sizeof(unsigned long long)) != cudaSuccess)
-    return bail(xb::fail(XB_E_CUDA, "cudaMemset failed"));
+  if (cudaMemsetAsync(r->stats, 0, STAT_COUNT * sizeof(unsigned long long), r->stream) != cudaSuccess)
+    return bail(xb::fail(XB_E_CUDA, "cudaMemsetAsync failed"));
   *out = r;
   return XB_OK;
 }
@@ -2531,7 +2532,8 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
       cap = up.big_leaves;
     }
     if (first > 0)
-      CK(cudaMemcpy(const_cast<uint2*>(sc.big_leaves), big_leaves.data(), first * sizeof(uint2), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(const_cast<uint2*>(sc.big_leaves), big_leaves.data(), first * sizeof(uint2),
+                         cudaMemcpyHostToDevice, r->stream));
   }
   // ── analytic prims in PrimBLAS slot order ──
   std::vector<float4> pnodes, prims;
@@ -2639,10 +2641,12 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   sc.sun_nee = (r->cfg.flags & XB_FLAG_SUN_NEE) != 0;
   sc.loose_boxes = up.loose != 0;
   sc.watertight = (r->cfg.flags & XB_FLAG_WATERTIGHT) != 0;
+  std::vector<float> cdf;
   if ((r->cfg.flags & XB_FLAG_SKY_IS) && sc.sky_intensity > 0.f) {
-    std::vector<float> cdf;
     if (sky_table(sc, cdf) && (rc = dev_upload(r, cdf, &sc.sky_cdf))) return rc;
   }
+  // the other lanes' and the callers' streams read the scene without waiting for this one
+  CK(cudaStreamSynchronize(r->stream));
   r->scene_opaque = opaque;
   r->has_scene = true;
   return XB_OK;
@@ -2756,14 +2760,13 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   if (!pack_tlas(nodes.data(), (int)nodes.size(), (int)r->inst_geom.size(), tlas, big) ||
       (int64_t)nodes.size() > r->tlas_cap || (int64_t)big.size() > r->big_leaves)
     return set_err(r, XB_E_UNSUPPORTED, "xb_refit_mesh: the rebuilt TLAS does not fit the uploaded scene's");
-  if (!tlas.empty()) {
-    CK(cudaMemcpy(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice));
-  }
-  if (!order.empty()) {
-    const std::vector<DevInstance> ordered = in_tlas_order(r->inst_dev, order.data(), order.size());
-    CK(cudaMemcpy(const_cast<DevInstance*>(sc.inst), ordered.data(), ordered.size() * sizeof(DevInstance),
-                  cudaMemcpyHostToDevice));
-  }
+  const std::vector<DevInstance> ordered = in_tlas_order(r->inst_dev, order.data(), order.size());
+  if (!tlas.empty())
+    CK(cudaMemcpyAsync(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
+  if (!ordered.empty())
+    CK(cudaMemcpyAsync(const_cast<DevInstance*>(sc.inst), ordered.data(), ordered.size() * sizeof(DevInstance),
+                       cudaMemcpyHostToDevice, s));
+  CK(cudaStreamSynchronize(s));   // the other lanes' and the callers' streams do not wait for this one
   sc.num_tlas_nodes = (int32_t)nodes.size();
   bool moved = false;
   if (!nodes.empty()) {
