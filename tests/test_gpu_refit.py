@@ -57,3 +57,26 @@ def test_device_refit_refuses_light_meshes_and_bad_input():
     assert e.value.code == abi.XB_E_UNSUPPORTED
     with pytest.raises(xb.XenonError):
         r.refit_mesh(99, pos)
+
+
+@pytest.mark.parametrize("instances", [3, 14, 15, 40])
+def test_refit_whose_tlas_is_one_large_leaf(instances):
+    """Boxes whose areas overflow: the TLAS build then makes one leaf of all instances, at 15 or more
+    one that does not fit a stack entry."""
+    desc = scenes.icosphere_scene(level=2)
+    rng = np.random.default_rng(1)
+    desc.instances = [(0, (rng.normal(size=3) * 5).astype(np.float32), 1.0 + i / 20,
+                       (rng.random(3) * 360).astype(np.float32), i) for i in range(instances)]
+    host = HostScene.from_desc(desc)
+    r = _renderer(host)
+    pos = abi.view_arrays(host.view())["meshes"][0]["pos"]
+    huge = (pos * np.float32(1e18)).astype(np.float32)
+    rays = np.concatenate([scenes.random_rays((huge.min(0), huge.max(0)), 1 << 12, seed=2),
+                           scenes.random_rays((pos.min(0), pos.max(0)), 1 << 12, seed=3)])
+    for new in (huge, pos, huge):
+        r.refit_mesh(0, new)
+        host.refit_mesh(0, new)
+        got = r.trace_rays(rays)
+        assert (got["prim_id"] >= 0).mean() > 0.05
+        assert got.tobytes() == _renderer(host).trace_rays(rays).tobytes()
+    assert abi.view_arrays(host.view())["tlas_nodes"]["count"][0] == instances

@@ -201,7 +201,8 @@ struct xb_renderer {
   xb_bvh_node prim_root{};
   bool has_prim_root = false;
   int64_t tlas_cap = 0;         // TLAS nodes that fit at the front of the device's node array
-  int64_t big_leaves = 0;       // entries of its big_leaves
+  int64_t big_leaves = 0;       // entries of its big_leaves that the upload uses,
+  int64_t big_cap = 0;          // and that there is room for: a refit's TLAS uses the rest
   void* refit_mem = nullptr;
   size_t refit_bytes = 0;
 };
@@ -2488,7 +2489,8 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
     const uint32_t first = (uint32_t)big_leaves.size();
     uint32_t cap = first + (uint32_t)(slot_base / kEntryEscape) + 1;
     for (int turn = 0; turn < 2; ++turn) {
-      if ((rc = dev_array(r, cap, &sc.big_leaves))) return rc;
+      r->big_cap = (int64_t)cap + std::max(0, v->num_instances) / kEntryEscape;
+      if ((rc = dev_array(r, (size_t)r->big_cap, &sc.big_leaves))) return rc;
       up = UploadStatus{};
       up.big_leaves = first;
       CK(cudaMemcpyAsync(status, &up, sizeof(up), cudaMemcpyHostToDevice, r->stream));
@@ -2756,16 +2758,22 @@ int xb_refit_mesh(xb_renderer* r, int32_t mesh, const float* positions, const fl
   std::vector<float4> tlas;
   std::vector<uint2> big((size_t)r->big_leaves);
   DevScene& sc = r->scene;
-  // every leaf of this TLAS is one instance, so it fits the array and adds no big leaf
+  // a leaf of this TLAS holds one instance, or, where the boxes' areas overflow, any number; each
+  // instance is in one leaf, so the nodes and the big leaves fit their arrays
   if (!pack_tlas(nodes.data(), (int)nodes.size(), (int)r->inst_geom.size(), tlas, big) ||
-      (int64_t)nodes.size() > r->tlas_cap || (int64_t)big.size() > r->big_leaves)
+      (int64_t)nodes.size() > r->tlas_cap || (int64_t)big.size() > r->big_cap) {
+    r->has_scene = false;   // the mesh has moved, and its instances' boxes have not
     return set_err(r, XB_E_UNSUPPORTED, "xb_refit_mesh: the rebuilt TLAS does not fit the uploaded scene's");
+  }
   const std::vector<DevInstance> ordered = in_tlas_order(r->inst_dev, order.data(), order.size());
   if (!tlas.empty())
     CK(cudaMemcpyAsync(const_cast<float4*>(sc.nodes), tlas.data(), tlas.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
   if (!ordered.empty())
     CK(cudaMemcpyAsync(const_cast<DevInstance*>(sc.inst), ordered.data(), ordered.size() * sizeof(DevInstance),
                        cudaMemcpyHostToDevice, s));
+  if ((int64_t)big.size() > r->big_leaves)
+    CK(cudaMemcpyAsync(const_cast<uint2*>(sc.big_leaves) + r->big_leaves, big.data() + r->big_leaves,
+                       (big.size() - (size_t)r->big_leaves) * sizeof(uint2), cudaMemcpyHostToDevice, s));
   CK(cudaStreamSynchronize(s));   // the other lanes' and the callers' streams do not wait for this one
   sc.num_tlas_nodes = (int32_t)nodes.size();
   bool moved = false;
