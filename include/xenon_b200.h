@@ -309,6 +309,8 @@ typedef struct xb_config {
 int  xb_create(const xb_config *cfg, xb_renderer **out);
 void xb_destroy(xb_renderer *r);
 int  xb_last_error(const xb_renderer *r, char *buf, size_t len);
+/* Copies the scene to the device. Indices out of range are refused (XB_E_INVALID), and so is a TLAS
+ * in which a node lies below itself, whose walk might not end. */
 int  xb_upload_scene(xb_renderer *r, const xb_scene_view *view);
 /* Moves the vertices of uploaded mesh `mesh` and refits its BLAS on the device: the triangles
  * take the new positions, and every node box is recomputed bottom-up by one kernel in which the

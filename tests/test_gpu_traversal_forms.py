@@ -159,3 +159,57 @@ def test_records_at_4_byte_alignment(mode):
     r.sync()
     assert out[1:1 + len(rays) * 16].cpu().numpy().tobytes() == want.tobytes()
     assert int(out[0]) == 0 and not out[1 + len(rays) * 16:].any()
+
+
+def _below(nd, i):
+    """The nodes that the walk from node i reaches."""
+    seen, todo = set(), [int(i)]
+    while todo:
+        k = todo.pop()
+        if k in seen:
+            continue
+        seen.add(k)
+        if nd["count"][k] == 0:
+            todo += [int(nd["child"][k]), int(nd["child"][k]) + 1]
+    return seen
+
+
+def _axis(nd, i):
+    e = nd["mx"][i] - nd["mn"][i]
+    return 0 if e[0] > e[1] and e[0] > e[2] else (1 if e[1] > e[2] else 2)
+
+
+@pytest.mark.parametrize("kind", ["same_axis", "other_axis", "shifted", "many", "spare_nodes"])
+def test_tlas_nodes_that_share_children_match_the_oracle(kind):
+    """A TLAS whose nodes form no tree, but whose walk ends: a child pair with two parents (which
+    order it along the same axis, or along different ones), two pairs with one node in common,
+    many shared pairs, and nodes that no walk reaches."""
+    desc = scenes.instanced_grid(grid=6, levels=(2, 2, 3, 3), with_prims=True)
+    hs = HostScene.from_desc(desc)
+    v = hs.view()
+    n = v.num_tlas_nodes
+    nd = np.concatenate([_nodes(v.tlas_nodes, n).copy(), np.zeros(5, abi.NODE_DTYPE)])
+    nd["child"][n + 1:n + 3] = 1          # spare interior nodes, of which two share the root's children
+    rng = np.random.default_rng(3)
+    inner = np.nonzero(nd["count"][:n] == 0)[0]
+    shared = 0
+    if kind != "spare_nodes":
+        pairs = [(a, b) for a in inner[1:] for b in inner[1:] if a != b]
+        rng.shuffle(pairs)
+        for a, b in pairs:
+            c = int(nd["child"][b]) + (1 if kind == "shifted" else 0)
+            if c + 1 >= n or a in _below(nd, c) or a in _below(nd, c + 1) or c == nd["child"][a]:
+                continue
+            if kind == "same_axis" and _axis(nd, a) != _axis(nd, b):
+                continue
+            if kind == "other_axis" and _axis(nd, a) == _axis(nd, b):
+                continue
+            nd["child"][a] = c
+            shared += 1
+            if shared == (8 if kind == "many" else 1):
+                break
+        assert shared > 0
+    if kind == "spare_nodes":
+        v.num_tlas_nodes = len(nd)
+    v.tlas_nodes = nd.ctypes.data
+    _same(Renderer(16, 16), v, _rays(desc, 1 << 14, 21))

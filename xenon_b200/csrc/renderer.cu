@@ -1470,46 +1470,90 @@ float4 node_hi(const xb_bvh_node& n, uint32_t child) {
 
 // TLAS nodes as DevScene::nodes holds them (entries and keys: dev_scene.cuh). Leaves that an entry
 // cannot hold go to big_leaves, and so do, as empty ones, nodes whose children or instances do not
-// exist. False when a node has two parents (its pair's key would serve one of them) or is the
-// root's parent, or there are too many.
+// exist. A node stays at its index; but key and axis are its parent's view of it, so a pair of
+// children that a second parent orders along another axis, or one of which is in another pair, gets
+// a copy behind the nodes, one for every axis it is ordered along (at most one pair per interior
+// node). False when a walk from the root would not end, or there are too many nodes.
 bool pack_tlas(const xb_bvh_node* nodes, int32_t n, int32_t num_inst, std::vector<float4>& out,
                std::vector<uint2>& big_leaves) {
-  if (n >= (1 << 27)) return false;
+  out.clear();
+  if (n <= 0) return true;
+  constexpr int64_t kMaxNodes = 1 << 27;
+  if (n >= kMaxNodes) return false;
+  auto exists = [&](const xb_bvh_node& nd) {
+    return nd.count > 0 ? (int64_t)nd.child + nd.count <= num_inst : (int64_t)nd.child + 1 < n;
+  };
+  auto axis = [](const xb_bvh_node& nd) {   // tlas.cpp:221-226
+    const float ex = nd.mx[0] - nd.mn[0], ey = nd.mx[1] - nd.mn[1], ez = nd.mx[2] - nd.mn[2];
+    return (ex > ey && ex > ez) ? 0 : (ey > ez ? 1 : 2);
+  };
+  // the nodes that a walk reaches, in depth-first order; a node met below itself is a cycle
+  enum : uint8_t { NEW, OPEN, DONE };
+  std::vector<uint8_t> state(n, NEW);
+  std::vector<int32_t> todo{0}, reached;
+  while (!todo.empty()) {
+    const int32_t i = todo.back();
+    if (state[i] != NEW) {
+      state[i] = DONE;
+      todo.pop_back();
+      continue;
+    }
+    state[i] = OPEN;
+    reached.push_back(i);
+    if (nodes[i].count > 0 || !exists(nodes[i])) continue;
+    for (uint32_t c = nodes[i].child; c <= nodes[i].child + 1; ++c) {
+      if (state[c] == OPEN) return false;
+      if (state[c] == NEW) todo.push_back((int32_t)c);
+    }
+  }
+  // each reached node's own words, at its index, and where its children's pair lies
+  out.resize(2 * (size_t)n, make_float4(0.f, 0.f, 0.f, 0.f));
+  std::vector<uint8_t> taken(n, 0);
+  std::vector<int64_t> place(3 * (size_t)n, -1);   // of the pair (child, child + 1) ordered along an axis
   bool loose = false;
-  std::vector<uint32_t> entry(n);
-  std::vector<float> key(n, 0.f);
-  std::vector<uint8_t> seen(n, 0);
-  if (n > 0) seen[0] = 1;
-  for (int32_t i = 0; i < n; ++i) {
+  auto box = [&](size_t at, const xb_bvh_node& nd, uint32_t entry, float key) {
+    out[2 * at] = make_float4(nd.mn[0], nd.mn[1], nd.mx[0], nd.mx[1]);
+    out[2 * at + 1] = make_float4(nd.mn[2], nd.mx[2], u32_bits_to_f(entry), key);
+  };
+  std::vector<uint32_t> entry(n, 0);
+  std::vector<std::pair<uint32_t, int>> pairs;     // (child, axis) of every pair, as placed
+  taken[0] = 1;
+  for (const int32_t i : reached) {
     const xb_bvh_node& nd = nodes[i];
     for (int k = 0; k < 3; ++k) loose = loose || !(nd.mn[k] <= nd.mx[k]);
-    const bool leaf = nd.count > 0;
-    const bool exists = leaf ? (int64_t)nd.child + nd.count <= num_inst : (int64_t)nd.child + 1 < n;
-    if (exists && (!leaf || (nd.count < kEntryEscape && nd.child < (1u << 27)))) {
-      entry[i] |= (nd.count << 28) | (nd.child << 1);
-    } else {
+    const bool leaf = nd.count > 0, there = exists(nd);
+    if (!there || (leaf && (nd.count >= kEntryEscape || nd.child >= (1u << 27)))) {
       if (big_leaves.size() >= (1u << 27) - 1) return false;
-      entry[i] |= (kEntryEscape << 28) | ((uint32_t)big_leaves.size() << 1);
-      big_leaves.push_back(exists ? make_uint2(nd.child, nd.count) : make_uint2(0, 0));
+      entry[i] = (kEntryEscape << 28) | ((uint32_t)big_leaves.size() << 1);
+      big_leaves.push_back(there ? make_uint2(nd.child, nd.count) : make_uint2(0, 0));
+      continue;
     }
-    if (leaf || !exists) continue;
-    const float ex = nd.mx[0] - nd.mn[0], ey = nd.mx[1] - nd.mn[1], ez = nd.mx[2] - nd.mn[2];
-    const uint32_t ax = (ex > ey && ex > ez) ? 0 : (ey > ez ? 1 : 2);   // tlas.cpp:221-226
+    if (leaf) {
+      entry[i] = (nd.count << 28) | (nd.child << 1);
+      continue;
+    }
+    const int ax = axis(nd);
+    int64_t& at = place[3 * (size_t)nd.child + ax];
+    if (at < 0) {
+      if (!taken[nd.child] && !taken[nd.child + 1]) {
+        at = nd.child;
+        taken[nd.child] = taken[nd.child + 1] = 1;
+      } else {
+        at = (int64_t)out.size() / 2;
+        if (at + 2 > kMaxNodes) return false;
+        out.resize(out.size() + 4);
+      }
+      pairs.emplace_back(nd.child, ax);
+    }
+    entry[i] = (uint32_t)at << 1;
+  }
+  box(0, nodes[0], entry[0], loose ? 1.f : 0.f);
+  for (const auto& [child, ax] : pairs)
     for (uint32_t c = 0; c < 2; ++c) {
-      const uint32_t ch = nd.child + c;
-      if (seen[ch]) return false;
-      seen[ch] = 1;
-      key[ch] = (nodes[ch].mn[ax] + nodes[ch].mx[ax]) * 0.5f;
-      entry[ch] |= c == 0 ? (ax & 1u) : (ax >> 1);
+      const xb_bvh_node& nd = nodes[child + c];
+      box((size_t)place[3 * (size_t)child + ax] + c, nd, entry[child + c] | (uint32_t)(c == 0 ? ax & 1 : ax >> 1),
+          (nd.mn[ax] + nd.mx[ax]) * 0.5f);
     }
-  }
-  if (loose) key[0] = 1.f;
-  out.clear();
-  for (int32_t i = 0; i < n; ++i) {
-    const xb_bvh_node& nd = nodes[i];
-    out.push_back(make_float4(nd.mn[0], nd.mn[1], nd.mx[0], nd.mx[1]));
-    out.push_back(make_float4(nd.mn[2], nd.mx[2], u32_bits_to_f(entry[i]), key[i]));
-  }
   return true;
 }
 
@@ -2433,7 +2477,11 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   // ── the meshes' places in the device arrays: BLAS nodes odd-aligned per mesh, slot-ordered
   // triangles; the refit passes (refit_kernels.h, which states this layout) and the host refit's
   // packing read it too. The TLAS nodes come first; a refit's has at most two per instance ──
-  const int64_t tlas_cap = std::max<int64_t>(v->num_tlas_nodes, 2 * (int64_t)v->num_instances);
+  std::vector<uint2> big_leaves;
+  std::vector<float4> tlas;
+  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves))
+    return set_err(r, XB_E_INVALID, "a walk of the TLAS does not end, or it is too large");
+  const int64_t tlas_cap = std::max<int64_t>((int64_t)tlas.size() / 2, 2 * (int64_t)v->num_instances);
   std::vector<int32_t> root_of(v->num_meshes, -1);
   std::vector<DevMesh> meshes(v->num_meshes);
   r->mesh_layout.assign(v->num_meshes, xb_renderer::MeshLayout());
@@ -2464,10 +2512,6 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
   }
   if (node_count >= (1u << 28) || slot_base >= (1 << 28))
     return set_err(r, XB_E_UNSUPPORTED, "scene too large: more than 2^28 BLAS nodes or triangles");
-  std::vector<uint2> big_leaves;
-  std::vector<float4> tlas;
-  if (!pack_tlas(v->tlas_nodes, v->num_tlas_nodes, v->num_instances, tlas, big_leaves))
-    return set_err(r, XB_E_INVALID, "a TLAS node has two parents, or the TLAS is too large");
   DevScene& sc = r->scene;
   std::memset(&sc, 0, sizeof(sc));
   if ((rc = dev_array(r, 2 * (size_t)node_count, &sc.nodes))) return rc;
