@@ -62,3 +62,25 @@ def test_bad_indices_are_refused(what, level):
     r.upload_scene(HostScene.from_desc(desc))
     rays = scenes.random_rays(scenes.scene_bounds(desc), 256, seed=1)
     assert (r.trace_rays(rays)["prim_id"] >= 0).any()
+
+
+@pytest.mark.parametrize("level", [2, 6])
+@pytest.mark.parametrize("missing", ["ny", "nz"])
+def test_a_missing_normal_component_is_zero(missing, level):
+    """Normals of which one component's array is NULL: that component is 0, whatever device memory
+    held before (a scene with all three was uploaded by the same renderer)."""
+    desc = scenes.icosphere_scene(level=level)
+    desc.meshes[0].normals = desc.meshes[0].positions / np.linalg.norm(desc.meshes[0].positions, axis=1, keepdims=True)
+    rays = scenes.random_rays(scenes.scene_bounds(desc), 1 << 12, seed=3)
+    hs = HostScene.from_desc(desc)
+    v = hs.view()
+    r = Renderer(16, 16)
+    r.upload_scene(v)
+    zeros = np.zeros(v.meshes[0].num_vertices, np.float32)
+    setattr(v.meshes[0], missing, zeros.ctypes.data_as(ctypes.POINTER(ctypes.c_float)))
+    want, _ = port.PortScene(v).trace(rays, abi.XB_TRACE_CLOSEST)
+    setattr(v.meshes[0], missing, ctypes.POINTER(ctypes.c_float)())
+    r.upload_scene(v)
+    got = r.trace_rays(rays)
+    assert (got["prim_id"] >= 0).mean() > 0.1
+    assert got["normal"].tobytes() == want["normal"].tobytes()

@@ -2257,7 +2257,8 @@ UploadArgs mesh_blob(const xb_mesh_view& mv, const xb_renderer::MeshLayout& ml, 
   take(&a.indices, true, 12 * (size_t)ml.num_tris);
   take(&a.mat_ids, mv.mat_ids != nullptr, 4 * (size_t)ml.num_tris);
   for (int k = 0; k < 3; ++k) take(&a.v[k], true, 4 * (size_t)ml.num_verts);
-  for (int k = 0; k < 3; ++k) take(&a.n[k], mv.nx != nullptr, 4 * (size_t)ml.num_verts);
+  const float* const n[3] = {mv.nx, mv.nx ? mv.ny : nullptr, mv.nx ? mv.nz : nullptr};
+  for (int k = 0; k < 3; ++k) take(&a.n[k], n[k] != nullptr, 4 * (size_t)ml.num_verts);
   a.bytes = at;
   a.node_base = ml.node_base;
   a.slot_base = ml.slot_base;
@@ -2553,9 +2554,9 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
             {mv.indices, a.indices, 12 * (size_t)ml.num_tris}, {mv.mat_ids, a.mat_ids, 4 * (size_t)ml.num_tris},
             {mv.vx, a.v[0], 4 * (size_t)ml.num_verts}, {mv.vy, a.v[1], 4 * (size_t)ml.num_verts},
             {mv.vz, a.v[2], 4 * (size_t)ml.num_verts}, {mv.nx, a.n[0], 4 * (size_t)ml.num_verts},
-            {mv.nx ? mv.ny : nullptr, a.n[1], 4 * (size_t)ml.num_verts}, {mv.nx ? mv.nz : nullptr, a.n[2], 4 * (size_t)ml.num_verts}};
+            {mv.ny, a.n[1], 4 * (size_t)ml.num_verts}, {mv.nz, a.n[2], 4 * (size_t)ml.num_verts}};
         for (const auto& q : parts) {
-          if (!q.src || !q.bytes) continue;
+          if (!q.src || !q.dst || !q.bytes) continue;
           if (together) std::memcpy(host.data() + (static_cast<const char*>(q.dst) - static_cast<char*>(mem.p)), q.src, q.bytes);
           else CK(cudaMemcpyAsync(const_cast<void*>(q.dst), q.src, q.bytes, cudaMemcpyHostToDevice, r->stream));
         }
