@@ -84,3 +84,22 @@ def test_a_missing_normal_component_is_zero(missing, level):
     got = r.trace_rays(rays)
     assert (got["prim_id"] >= 0).mean() > 0.1
     assert got["normal"].tobytes() == want["normal"].tobytes()
+
+
+def test_instances_without_a_tlas_hit_nothing_until_a_refit_builds_one():
+    desc = scenes.instanced_grid(grid=3, levels=(3, 3, 3, 3), with_prims=True)
+    rays = scenes.random_rays(scenes.scene_bounds(desc), 1 << 12, seed=4)
+    hs = HostScene.from_desc(desc)
+    v = hs.view()
+    r = Renderer(16, 16)
+    r.upload_scene(v)
+    want = r.trace_rays(rays)
+    assert (want["prim_id"] >= 0).mean() > 0.1
+    lit = {l[0] for l in desc.lights}
+    mesh = next(m for m in range(len(desc.meshes)) if m not in lit)
+    pos = abi.view_arrays(v)["meshes"][mesh]["pos"]
+    v.num_tlas_nodes = 0
+    r.upload_scene(v)
+    assert (r.trace_rays(rays)["prim_id"] < 0).all()
+    r.refit_mesh(mesh, pos)
+    assert r.trace_rays(rays).tobytes() == want.tobytes()

@@ -2629,9 +2629,10 @@ int xb_upload_scene(xb_renderer* r, const xb_scene_view* v) {
     }
   }
   r->inst_dev = insts;
+  // (without a TLAS in any order: a refit builds one)
   const std::vector<DevInstance> ordered =
-      in_tlas_order(insts, v->tlas_inst_indices, v->num_tlas_nodes > 0 ? v->num_instances : 0);
-  if (v->num_tlas_nodes > 0 && ordered.empty() && v->num_instances > 0)
+      v->num_tlas_nodes > 0 ? in_tlas_order(insts, v->tlas_inst_indices, v->num_instances) : insts;
+  if (ordered.size() != insts.size())
     return set_err(r, XB_E_INVALID, "TLAS instance index out of range");
   // ── materials, emitters, sky ──
   std::vector<DevMaterial> mats;
