@@ -102,6 +102,20 @@ def parse():
     return ap.parse_args()
 
 
+CLOSEST_KERNEL = "extend_persistent_kernel"   # the kernel of the roofline's closest-hit rays
+
+
+def profiled_dram_bytes_per_ray(path: str = os.path.join(ROOT, "profiles", f"{CLOSEST_KERNEL}_config2.json")):
+    """DRAM bytes per closest-hit ray of CLOSEST_KERNEL from its committed profile; None when there
+    is none or it measured another kernel."""
+    if not os.path.exists(path):
+        return None
+    with open(path) as f:
+        prof = json.load(f)
+    measured = prof.get("kernel", "").split("<")[0].split(" ")[0]
+    return prof.get("dram_bytes_per_closest_ray") if measured == CLOSEST_KERNEL else None
+
+
 def load_peaks() -> dict:
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -923,13 +937,8 @@ def main():
     ext_busy_ms = prof.extend_busy_ms
     achieved = ext_bytes / (ext_busy_ms * 1e-3) / 1e9
     step_avg = ext_bytes / n_prof / (t_max / args.steps * 1e-3) / 1e9
-    traffic = None
-    tp = os.path.join(ROOT, "profiles", "extend_kernel_config2.json")
-    if os.path.exists(tp):
-        with open(tp) as f:
-            tj = json.load(f)
-        if tj.get("dram_bytes_per_closest_ray"):
-            traffic = tj["dram_bytes_per_closest_ray"] * pst.rays_closest / max(prof.extend_launches, 1)
+    per_ray = profiled_dram_bytes_per_ray()
+    traffic = None if per_ray is None else per_ray * pst.rays_closest / max(prof.extend_launches, 1)
     # the same kernel with one wave in flight (untimed pass): its launches then have the GPU to
     # themselves, while in the timed region the other lanes' kernels run beside them
     lanes = r.tuning()["waves"]
@@ -950,7 +959,7 @@ def main():
         r.set_tuning(waves=lanes)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-                "peak_source": peaks["source"], "kernel": "extend_persistent_kernel (closest-hit traversal)",
+                "peak_source": peaks["source"], "kernel": f"{CLOSEST_KERNEL} (closest-hit traversal)",
                 "algorithmic_bytes_per_ray": ext_bytes_per_ray,
                 "algorithmic_bytes_per_launch": ext_bytes / max(prof.extend_launches, 1),
                 "extend_busy_ms_per_step": ext_busy_ms / n_prof,

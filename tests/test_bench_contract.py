@@ -67,3 +67,18 @@ def test_reference_arm_loads_no_library_of_this_package(ref):
     assert p.returncode == 0, p.stderr
     res = json.loads(p.stdout.strip().splitlines()[-1])
     assert res == {"loaded": False, "ref": True, "same_config": True}, res
+
+
+def test_roofline_traffic_is_the_timed_kernels(tmp_path):
+    """The DRAM bytes per ray that the roofline scales were measured on the kernel it names, which
+    the renderer has; a profile of another kernel gives none."""
+    import bench
+    src = open(os.path.join(ROOT, "xenon_b200", "csrc", "renderer.cu")).read()
+    assert f" {bench.CLOSEST_KERNEL}(DevScene" in src
+    assert bench.profiled_dram_bytes_per_ray() > 0
+    p = tmp_path / "p.json"
+    for kernel, want in (("extend_kernel<0, 0> (closest hit)", None), (bench.CLOSEST_KERNEL + "<0, 0> (closest hit)", 7.5),
+                         ("", None)):
+        p.write_text(json.dumps({"kernel": kernel, "dram_bytes_per_closest_ray": 7.5}))
+        assert bench.profiled_dram_bytes_per_ray(str(p)) == want
+    assert bench.profiled_dram_bytes_per_ray(str(tmp_path / "absent.json")) is None
