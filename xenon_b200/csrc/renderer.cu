@@ -156,12 +156,12 @@ struct xb_renderer {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
   int grid_ext = 0, grid_shade = 0, grid_shadow = 0, block = 128;
-  int grid_pext = 0, grid_pshadow = 0;
   bool thread_per_ray = false;   // XB_FLAG_THREAD_PER_RAY: one ray per thread traversal kernels
   int refill = 8;                // persistent traversal: refill a warp when this many lanes idle
   int ext_persistent_from = 0;   // bounces >= this trace closest hits with persistent warps
   bool shadow_persistent = true;
-  int occ_pext = 1, occ_pshadow = 1;  // blocks of the persistent kernels that fit on an SM at once
+  // blocks of the persistent kernels that fit on an SM at once, by form: [shared stack][counting]
+  int occ_pext[2][2] = {{1, 1}, {1, 1}}, occ_pshadow[2][2] = {{1, 1}, {1, 1}};
   int occ_api[2] = {1, 1};   // trace_api_persistent_kernel<closest / any>
   int stack_sh = 0;             // BLAS stack entries in shared memory (tuning shared_stack)
   xb_tuning tune{};
@@ -1645,13 +1645,11 @@ int apply_tuning(xb_renderer* r, const xb_tuning& t) {
   r->shadow_persistent = c.shadow_persistent == 1;
   r->refill = c.refill;
   // Persistent kernels (their blocks loop until the queue is empty) launch at most the blocks
-  // that fit at once; the others fetch warps of work from a counter or take tiles in a
+  // that fit at once (trace_grid.h); the others fetch warps of work from a counter or take tiles in a
   // grid-stride loop, so blocks beyond the resident ones queue and, as they start while others
   // retire, interleave with the other wave lane's kernels.
   r->grid_ext = r->num_sms * c.extend_blocks_per_sm;
-  r->grid_pext = r->num_sms * std::min(r->occ_pext, c.extend_blocks_per_sm);
   r->grid_shadow = r->num_sms * c.shadow_blocks_per_sm;
-  r->grid_pshadow = r->num_sms * std::min(r->occ_pshadow, c.shadow_blocks_per_sm);
   r->grid_shade = r->num_sms * c.shade_blocks_per_sm;
   r->grid_gshade = r->num_sms * std::min(r->occ_gshade, c.shade_blocks_per_sm);
   const int64_t npix = (int64_t)r->cfg.width * r->cfg.height;
@@ -1766,8 +1764,8 @@ void launch_extend_k(xb_renderer* r, const LaneRef& L, int d, bool count) {
   TraceQueue tq{w.ray_o[q], w.ray_d[q], cd_ + CNT_RAYS, cd_ + CNT_FETCH_EXT, w.hit, w.hit_inst,
                 nullptr, nullptr, r->stats, 0};
   auto kern = count ? extend_persistent_kernel<true, kSh> : extend_persistent_kernel<false, kSh>;
-  kern<<<per_thread ? r->grid_ext : r->grid_pext, 128, smem, L.s>>>(r->scene, tq, per_thread ? 32 : r->refill,
-                                                                   r->num_sms * r->occ_pext * 4);
+  const xb::TraceGrid g = xb::trace_grid(r->grid_ext, r->num_sms, r->occ_pext[kSh > 0][count], per_thread);
+  kern<<<g.blocks, 128, smem, L.s>>>(r->scene, tq, per_thread ? 32 : r->refill, g.warps);
 }
 
 void launch_extend(xb_renderer* r, const LaneRef& L, int d, bool count) {
@@ -1786,8 +1784,8 @@ void launch_shadow_k(xb_renderer* r, const LaneRef& L, int d, int k, bool count,
                 cd_ + (k ? CNT_FETCH_SH_SUN : CNT_FETCH_SH_AREA), nullptr, nullptr, w.sh_c[k], w.L,
                 r->stats, r->tune.shadow_order == 2};
   auto kern = count ? shadow_persistent_kernel<true, kSh> : shadow_persistent_kernel<false, kSh>;
-  kern<<<per_thread ? r->grid_shadow : r->grid_pshadow, 128, smem, s>>>(r->scene, tq, per_thread ? 32 : r->refill,
-                                                                       r->num_sms * r->occ_pshadow * 4);
+  const xb::TraceGrid g = xb::trace_grid(r->grid_shadow, r->num_sms, r->occ_pshadow[kSh > 0][count], per_thread);
+  kern<<<g.blocks, 128, smem, s>>>(r->scene, tq, per_thread ? 32 : r->refill, g.warps);
 }
 
 void launch_shadows(xb_renderer* r, const LaneRef& L, int d, bool count, cudaStream_t s) {
@@ -2387,10 +2385,21 @@ int xb_create(const xb_config* cfg, xb_renderer** out) {
     const int by_smem = smem_sm / std::max<int>(1, (int)(kGuidedShadeSmem + fa.sharedSizeBytes) + smem_rsv);
     r->occ_gshade = std::max(1, std::min(4, std::min(by_regs, by_smem)));
   }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extend_persistent_kernel<false, 0>, 128, 0);
-  r->occ_pext = std::max(occ, 1);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shadow_persistent_kernel<false, 0>, 128, 0);
-  r->occ_pshadow = std::max(occ, 1);
+  {
+    using Kern = void (*)(DevScene, TraceQueue, int, int);
+    const Kern ext[2][2] = {{extend_persistent_kernel<false, 0>, extend_persistent_kernel<true, 0>},
+                            {extend_persistent_kernel<false, kSharedStack>, extend_persistent_kernel<true, kSharedStack>}};
+    const Kern sh[2][2] = {{shadow_persistent_kernel<false, 0>, shadow_persistent_kernel<true, 0>},
+                           {shadow_persistent_kernel<false, kSharedStack>, shadow_persistent_kernel<true, kSharedStack>}};
+    for (int k = 0; k < 2; ++k)
+      for (int c = 0; c < 2; ++c) {
+        const size_t smem = k ? (size_t)kSharedStack * kShStride * sizeof(uint32_t) : 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ext[k][c], 128, smem);
+        r->occ_pext[k][c] = std::max(occ, 1);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh[k][c], 128, smem);
+        r->occ_pshadow[k][c] = std::max(occ, 1);
+      }
+  }
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_api_persistent_kernel<false>, 128, 0);
   r->occ_api[0] = std::max(occ, 1);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_api_persistent_kernel<true>, 128, 0);

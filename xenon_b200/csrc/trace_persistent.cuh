@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "dev_scene.cuh"
+#include "trace_grid.h"
 
 namespace xbd {
 
@@ -60,8 +61,8 @@ struct TraceQueue {
 //                           (warp-uniform: every lane calls it with the same k)
 //   load<kAny>(ray, o, d, tmin, tmax), finish_any(ray, occluded),
 //   finish_closest(sc, ray, o, d, tmin, tmax, h), stats()
-// A queue shorter than the lanes of the warps that fit on the GPU at once is spread over all of
-// those warps: a warp's time is the union of what its lanes do, one kind of work after the other,
+// A queue shorter than the lanes of the launch's warps that fit on the GPU at once is spread over all
+// of those warps (trace_grid.h): a warp's time is the union of what its lanes do, one kind of work after the other,
 // so 8 rays on each of four warps are done sooner than 32 on one. That is most bounces of a path:
 // ms per sample at 1920x1080, closest / any hits, 261 instances 4.76 / 2.90 -> 4.05 / 2.43, one
 // instance 1.25 / 0.95 -> 1.12 / 0.87; a 256x256 sample in a box 0.276 / 0.203 -> 0.235 / 0.185
@@ -73,7 +74,7 @@ struct QueueIO {
   int n, per_warp;
   bool first;
   __device__ __forceinline__ QueueIO(const TraceQueue& tq, int warps)
-      : q(tq), n(*tq.count), per_warp(min(32, max(1, (n + warps - 1) / warps))), first(true) {}
+      : q(tq), n(*tq.count), per_warp(xb::queue_lanes(n, warps)), first(true) {}
   __device__ __forceinline__ int end() const { return n; }
   __device__ __forceinline__ int lanes() const { return per_warp; }
   __device__ __forceinline__ int grab(int lane, int leader, int k) {
