@@ -306,6 +306,11 @@ typedef struct xb_config {
   int32_t block_size;                /* threads per block of the trace kernels; 0 = automatic */
 } xb_config;
 
+/* Besides its scene, framebuffers and ray queues a renderer keeps, until xb_destroy: page-locked host
+ * memory of 1 MB; device scratch for the calls that wait for their work (xb_trace_rays,
+ * xb_render_views, xb_output_stage, xb_upload_scene), as large as the largest of them needed, 64 MB at
+ * most (a call that needs more allocates and frees its own); and xb_refit_mesh's scratch (12 to 24
+ * bytes a vertex and 8 a node of the largest mesh refitted). */
 int  xb_create(const xb_config *cfg, xb_renderer **out);
 void xb_destroy(xb_renderer *r);
 int  xb_last_error(const xb_renderer *r, char *buf, size_t len);

@@ -14,7 +14,7 @@ two passes), and keeps the fastest setting:
   guided_form                    guided bounce as a bounce kernel + network pass, or one fused kernel
                                  (searched for guided workloads only)
   shade_occupancy                blocks per SM the shading kernels are compiled to fit (registers)
-  shared_stack                   BLAS stack entries per thread kept in shared memory (1: none, 16)
+  shared_stack                   words of each thread's traversal stack in shared memory (1: none, 16)
   pixel_order                    camera rays in scanline order or in 8x4 pixel tiles per warp
   refill                         idle lanes that trigger a warp refill
   extend/shadow/shade_blocks_per_sm   blocks per SM in the grids (persistent kernels: at most

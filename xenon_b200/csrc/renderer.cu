@@ -163,7 +163,7 @@ struct xb_renderer {
   // blocks of the persistent kernels that fit on an SM at once, by form: [shared stack][counting]
   int occ_pext[2][2] = {{1, 1}, {1, 1}}, occ_pshadow[2][2] = {{1, 1}, {1, 1}};
   int occ_api[2] = {1, 1};   // trace_api_persistent_kernel<closest / any>
-  int stack_sh = 0;             // BLAS stack entries in shared memory (tuning shared_stack)
+  int stack_sh = 0;             // words of a thread's traversal stack in shared memory (tuning shared_stack)
   xb_tuning tune{};
   // profiling
   int prof_flags = 0;
@@ -646,9 +646,11 @@ constexpr size_t kGuidedShadeSmem =
 // there is no network, shared memory or barrier, so it launches like the plain bounce.
 // Its code and the network pass's were 455 and 210 KB before the passes around one evaluation (see
 // dev_bsdf.cuh). B200, both kernels, ms per sample at 1080p / 720p: 261 instances of every material
-// kind 4.05 -> 1.61, the room of one diffuse material 1.28 -> 1.23; the fused form, whose atomics
-// now lie on a tile's serial chain, 1.48 -> 1.82 in the room and 6.4 -> 3.4 (whole render) with the
-// instances.
+// kind 4.05 -> 1.61, the room of one diffuse material 1.28 -> 1.23; the fused form's kernel alone,
+// whose atomics now lie on a tile's serial chain, 1.48 -> 1.82 in the room. Whole renders of four
+// samples, before those passes and the traversal's -> now, default launch settings, untrained
+// network: two-kernel form 4.32 -> 2.66 (room) and 12.1 -> 5.46 (instances), fused 4.75 -> 3.48 and
+// 18.4 -> 8.12.
 template <bool kNet, int kOcc>
 __global__ void __launch_bounds__(128, kNet ? 4 : kOcc) guided_shade_kernel(ShadeArgs a, GuideShadeArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -1750,8 +1752,8 @@ LaneRef lane_ref(xb_renderer* r, int k) {
   return LaneRef{&x.wb, x.s, x.s2, x.ev_shade, x.ev_shadow};
 }
 
-// The traversal kernels come in two forms: the BLAS stack wholly in local memory (kSh = 0), or
-// its first kSharedStack entries in shared memory (tuning shared_stack).
+// The traversal kernels come in two forms: the stack wholly in local memory (kSh = 0), or its first
+// kSharedStack words in shared memory (tuning shared_stack).
 
 // One ray per thread is the same kernel with every lane idle before a refill, on a grid of its own.
 template <int kSh>

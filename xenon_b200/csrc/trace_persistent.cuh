@@ -28,7 +28,9 @@
 // later; one that hits carries its entry distance on the stack, and its test at the pop is that
 // distance against the hit by then, the only term of the reference's test that has changed.
 // Any-hit rays (kAny) only need *whether* some triangle lies in [tmin, tmax], which does not depend
-// on order, so they descend nearest child first to find occluders sooner.
+// on order: shadow rays descend farther child first by default (they start on a surface, among boxes
+// that do not occlude them: 1-8 % per sample), ray queries nearer first (1 M uniform rays on 261
+// instances 397 us, farther first 461).
 #pragma once
 
 #include <type_traits>

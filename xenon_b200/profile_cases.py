@@ -14,7 +14,7 @@
                                                             one wave (2,073,600 paths, one lane, direct
                                                             launches; under 1 GB of queues): every
                                                             kernel of a bounce at its full size; SS = 16
-                                                            keeps 16 BLAS stack entries in shared memory
+                                                            keeps 16 traversal-stack words in shared memory
     python -m xenon_b200.profile_cases trace_uniform [N]    2^N (default 22) incoherent rays on the config-2
                                                             scene through xb_trace_rays_device, closest
                                                             then any hit
